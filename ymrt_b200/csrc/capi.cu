@@ -61,22 +61,6 @@ struct DeviceBuffer {
   }
 };
 
-std::vector<uint32_t> first_primes(int n) {
-  std::vector<uint32_t> p;
-  for (uint32_t c = 2; (int)p.size() < n; ++c) {
-    bool prime = true;
-    for (uint32_t q : p) {
-      if (q * q > c) break;
-      if (c % q == 0) {
-        prime = false;
-        break;
-      }
-    }
-    if (prime) p.push_back(c);
-  }
-  return p;
-}
-
 }  // namespace
 
 struct ymrt_context {
@@ -108,7 +92,6 @@ struct ymrt_context {
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   bool profiling = false;
   cudaEvent_t ev_stage[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  std::vector<uint32_t> primes, prime_sums;
   WaveCounters batch_counters{};  // frame totals across the launch groups of one batch
   // wave options (ymrt_set_option)
   bool sort_hits = true;
@@ -289,7 +272,7 @@ class SlotLease {
   bool ok() const { return ok_; }
   const uint32_t* slots() const { return slots_; }
   uint32_t slot(size_t k) const { return slots_[k]; }
-  // Uploads scenes[k] into the k-th leased slot (and the prime tables).
+  // Uploads scenes[k] into the k-th leased slot.
   cudaError_t upload(const DeviceScene* scenes, uint32_t n) const;
 
  private:
@@ -434,7 +417,7 @@ SlotLease::~SlotLease() {
 
 cudaError_t SlotLease::upload(const DeviceScene* scenes, uint32_t n) const {
   if (!ok_ || n > n_) return cudaErrorInvalidValue;
-  return upload_constants(scenes, slots_, n, ctx_->primes.data(), ctx_->prime_sums.data(), ctx_->stream);
+  return upload_constants(scenes, slots_, n, ctx_->stream);
 }
 
 }  // namespace
@@ -469,13 +452,6 @@ int ymrt_create(int device_ordinal, ymrt_context** out) {
   if ((e = cudaMallocHost(&ctx->ctl_host, sizeof(WaveControl))) != cudaSuccess)
     return ctx->cuda_fail(e, "cudaMallocHost");
   if ((e = ctx->counters_buf.ensure(sizeof(WaveCounters))) != cudaSuccess) return ctx->cuda_fail(e, "cudaMalloc");
-  ctx->primes = first_primes(kHaltonDims);
-  ctx->prime_sums.resize(kHaltonDims);
-  uint32_t acc = 0;
-  for (int i = 0; i < kHaltonDims; ++i) {
-    ctx->prime_sums[i] = acc;
-    acc += ctx->primes[i];
-  }
   *out = ctx.release();
   return YMRT_OK;
 }
@@ -724,10 +700,9 @@ int ymrt_scene_upload(ymrt_context* ctx, const ymrt_host_scene* hs, const uint32
                       ymrt_scene** out) {
   if (!ctx || !hs || !out || !halton_perm) return YMRT_ERR_INVALID;
   *out = nullptr;
-  size_t need = 0;
-  for (uint32_t p : ctx->primes) need += p;
-  if (perm_len != need)
-    return ctx->fail(YMRT_ERR_INVALID, "halton permutation table must hold " + std::to_string(need) + " entries");
+  if (perm_len != kHaltonTableSize)
+    return ctx->fail(YMRT_ERR_INVALID,
+                     "halton permutation table must hold " + std::to_string(kHaltonTableSize) + " entries");
   const HostScene& s = hs->s;
   cudaSetDevice(ctx->device);
   std::unique_ptr<ymrt_scene> sc(new (std::nothrow) ymrt_scene());

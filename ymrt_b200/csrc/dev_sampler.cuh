@@ -9,10 +9,51 @@
 
 namespace ym {
 
-// First 1000 primes and their prefix sums (offset of each prime's digit
-// permutation in the table), uploaded before each launch sequence.
-static __constant__ uint32_t c_primes[kHaltonDims];
-static __constant__ uint32_t c_prime_sums[kHaltonDims];
+// One Halton dimension: its prime base, the offset of the base's digit
+// permutation in the table, the multiplier of the exact division by the base
+// and 1 / base in float. In global memory, 16 bytes a dimension: the lanes of
+// a warp draw different dimensions (their paths are at different depths), and
+// a constant-bank read would replay once per distinct dimension.
+struct alignas(16) HaltonDim {
+  uint32_t base, offset, magic;
+  float inv_base;
+};
+struct HaltonTable {
+  HaltonDim dim[kHaltonDims];
+};
+// ceil(log2(base)) for a base of 2 or more.
+YM_HD constexpr uint32_t ceil_log2(uint32_t base) {
+  uint32_t l = 0;
+  while ((1u << l) < base) ++l;
+  return l;
+}
+constexpr HaltonTable make_halton_table() {
+  HaltonTable t{};
+  bool composite[7920] = {};  // the 1000th prime is 7919
+  uint32_t n = 0, sum = 0;
+  for (uint32_t c = 2; c < 7920 && n < (uint32_t)kHaltonDims; ++c) {
+    if (composite[c]) continue;
+    for (uint32_t q = c * c; q < 7920; q += c) composite[q] = true;
+    // m' = floor(2^32 (2^l - d) / d) + 1 with l = ceil(log2 d)
+    const uint64_t l2 = 1ull << ceil_log2(c);
+    t.dim[n].base = c;
+    t.dim[n].offset = sum;
+    t.dim[n].magic = (uint32_t)(((l2 - c) << 32) / c + 1ull);
+    t.dim[n].inv_base = 1.0f / float(c);
+    sum += c;
+    ++n;
+  }
+  return t;
+}
+static __device__ const HaltonTable g_halton = make_halton_table();
+
+// n / base for any 32-bit n, from the base's multiplier (Granlund and
+// Montgomery, "Division by Invariant Integers using Multiplication", PLDI
+// 1994, figure 4.1; shift = ceil(log2 base) - 1).
+__device__ __forceinline__ uint32_t divide_by_base(uint32_t n, uint32_t magic, uint32_t shift) {
+  const uint32_t t = __umulhi(n, magic);
+  return (t + ((n - t) >> 1)) >> shift;
+}
 
 // Evaluation order of the reference's multi-draw argument lists
 // (e.g. SampleLi(..., random(), random(), ...) at src/Shading.cu:325): the
@@ -60,39 +101,32 @@ __device__ __forceinline__ uint64_t halton_index(const DeviceScene& S, int px, i
 // RadicalInversion with a digit permutation, src/RandomSampler.cuh:462-480.
 // Indices below 2^32 (every sample of a 4K frame at 64 spp) take the 32-bit
 // division path; the digits, and therefore the result, are identical.
-__device__ __forceinline__ float radical_inverse_perm(uint64_t index, uint32_t base, const uint32_t* __restrict__ perm) {
-  const float inv_base = 1.0f / float(base);
+__device__ __forceinline__ float radical_inverse_perm(uint64_t index, const HaltonDim& D,
+                                                      const uint32_t* __restrict__ table) {
+  const uint32_t base = D.base;
+  const float inv_base = D.inv_base;
+  const uint32_t* __restrict__ perm = table + D.offset;
   uint64_t radical_sum = 0;
   float base_multiply = 1.0f;
-  if (index <= 0xFFFFFFFFull) {
-    uint32_t idx = (uint32_t)index;
-    while (idx) {
-      const uint32_t next = idx / base;
-      const uint32_t digit = idx - next * base;
-      radical_sum = radical_sum * base + __ldg(perm + digit);
-      base_multiply *= inv_base;
-      idx = next;
-    }
-  } else {
-    while (index) {
-      const uint64_t next = index / base;
-      const uint64_t digit = index - next * base;
-      radical_sum = radical_sum * base + __ldg(perm + digit);
-      base_multiply *= inv_base;
-      index = next;
-    }
+#pragma unroll 1
+  while (index > 0xFFFFFFFFull) {
+    const uint64_t next = index / base;
+    const uint64_t digit = index - next * base;
+    radical_sum = radical_sum * base + __ldg(perm + digit);
+    base_multiply *= inv_base;
+    index = next;
+  }
+  uint32_t idx = (uint32_t)index;
+  const uint32_t shift = 31u - (uint32_t)__clz((int)(base - 1u));  // ceil(log2 base) - 1
+  while (idx) {
+    const uint32_t next = divide_by_base(idx, D.magic, shift);
+    const uint32_t digit = idx - next * base;
+    radical_sum = radical_sum * base + __ldg(perm + digit);
+    base_multiply *= inv_base;
+    idx = next;
   }
   const float postfix_zero = (float)__ldg(perm) * base_multiply * inv_base / (1.0f - inv_base);
   return gmax(0.000001f, gmin(__ull2float_rn(radical_sum) * base_multiply + postfix_zero, 0.999999f));
-}
-
-// HaltonSampler::Random1D, src/RandomSampler.cuh:430-439.
-__device__ __forceinline__ float halton_draw(PathSampler& s, const uint32_t* __restrict__ table) {
-  const uint32_t d = s.dim;
-  const float r = radical_inverse_perm(s.index, c_primes[d], table + c_prime_sums[d]);
-  ++s.dim;
-  if (s.dim >= (uint32_t)kHaltonDims) s.dim = 2;
-  return r;
 }
 
 // The 4-D PCG hash of Jarzynski and Olano, "Hash Functions for GPU
@@ -121,9 +155,8 @@ __device__ __forceinline__ uint4 pcg4d(uint4 v) {
 
 // PCGSampler::Random1D (src/RandomSampler.cuh:400-405): hash of (pixel,
 // dimension, sample in pixel, frame), first lane over 2^32.
-__device__ __forceinline__ float pcg_draw(PathSampler& s) {
+__device__ __forceinline__ float pcg_draw(const PathSampler& s) {
   const uint4 h = pcg4d(make_uint4((uint32_t)s.index, s.dim, (uint32_t)(s.index >> 32), s.aux));
-  ++s.dim;
   return (float)h.x / 4294967296.0f;
 }
 
@@ -155,7 +188,7 @@ __device__ __forceinline__ uint32_t owen_scramble(uint32_t v, uint32_t dim, uint
 // SobolSampler::Random1D / SobolSample (src/RandomSampler.cuh:533-612): the
 // Gray-code-ordered Sobol point of the sample in this dimension (generator
 // matrices are an input: 32 columns per dimension), Owen-scrambled, clamped.
-__device__ __forceinline__ float sobol_draw(PathSampler& s, const uint32_t* __restrict__ matrices) {
+__device__ __forceinline__ float sobol_draw(const PathSampler& s, const uint32_t* __restrict__ matrices) {
   const uint32_t dim = s.dim;
   const uint32_t* m = matrices + (size_t)dim * 32u;
   const uint32_t index = (uint32_t)s.index;
@@ -163,17 +196,35 @@ __device__ __forceinline__ float sobol_draw(PathSampler& s, const uint32_t* __re
   for (uint32_t i = index ^ (index >> 1), j = 0; i; i >>= 1, ++j)
     if (i & 1u) v ^= __ldg(m + j);
   v = owen_scramble(v, dim, (uint32_t)(s.index >> 32));
-  const float r = gmax(0.000001f, gmin(float(v) / float(0xFFFFFFFFu), 0.999999f));
-  ++s.dim;
-  if (s.dim >= 4096u) s.dim = 1;  // the reference wraps here (and prints a warning)
-  return r;
+  return gmax(0.000001f, gmin(float(v) / float(0xFFFFFFFFu), 0.999999f));
 }
 
-// RandomSampler::Random1D (src/RandomSampler.cuh:681-697).
+// The sample of the state's current dimension. One out-of-line copy per
+// kernel: the shading kernels are bound by instruction fetch, and the three
+// samplers' loops inlined at each draw site were 50-107 KB of their 275-707 KB
+// of code. With the multiplier division, one B200: volumetric 1280x720 16 spp
+// 579 -> 514 ms, image textures 640x480 16 spp 43.3 -> 38.0 ms, solid textures
+// 1280x720 8 spp 192 -> 181 ms, instanced 1080p 64 spp 298 -> 294 ms.
+static __device__ __noinline__ float sampler_value(PathSampler s, uint32_t sampler_type,
+                                                   const uint32_t* __restrict__ table) {
+  if (sampler_type == kSamplerHalton) return radical_inverse_perm(s.index, g_halton.dim[s.dim], table);
+  if (sampler_type == kSamplerPcg) return pcg_draw(s);
+  return sobol_draw(s, table);
+}
+
+// RandomSampler::Random1D (src/RandomSampler.cuh:681-697), with the
+// dimension's wrap of HaltonSampler::Random1D (:430-439) and
+// SobolSampler::Random1D (:533-545).
 __device__ __forceinline__ float sample1d(PathSampler& s, const DeviceScene& S) {
-  if (S.sampler_type == kSamplerHalton) return halton_draw(s, S.halton_perm);
-  if (S.sampler_type == kSamplerPcg) return pcg_draw(s);
-  return sobol_draw(s, S.sobol_matrices);
+  const uint32_t type = S.sampler_type;
+  const float r = sampler_value(s, type, type == kSamplerHalton ? S.halton_perm : S.sobol_matrices);
+  ++s.dim;
+  if (type == kSamplerHalton) {
+    if (s.dim >= (uint32_t)kHaltonDims) s.dim = 2;
+  } else if (type == kSamplerSobol) {
+    if (s.dim >= 4096u) s.dim = 1;  // the reference wraps here (and prints a warning)
+  }
+  return r;
 }
 
 // Two / three draws bound to argument positions in the reference's order.

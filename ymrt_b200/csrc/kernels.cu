@@ -431,16 +431,19 @@ __global__ void k_debug_halton(uint32_t slot, int n, const int* px, const int* p
   offset[2 * i] = gmin(gmax(ox, 0.000001f), 0.999999f);
   offset[2 * i + 1] = gmin(gmax(oy, 0.000001f), 0.999999f);
   PathSampler hs{idx, 2u, 0u};
-  for (int d = 0; d < n_dims; ++d) dims[(size_t)i * n_dims + d] = halton_draw(hs, S.halton_perm);
+  for (int d = 0; d < n_dims; ++d) {
+    dims[(size_t)i * n_dims + d] = sampler_value(hs, kSamplerHalton, S.halton_perm);
+    if (++hs.dim >= (uint32_t)kHaltonDims) hs.dim = 2;
+  }
 }
 
 // ------------------------------------------------------------ launchers ---
 
-cudaError_t upload_constants(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, const uint32_t* primes,
-                             const uint32_t* prime_sums, cudaStream_t stream) {
-  cudaError_t e = upload_slots_here(scenes, slots, n, primes, prime_sums, stream);
-  if (e == cudaSuccess) e = upload_slots_media(scenes, slots, n, primes, prime_sums, stream);
-  if (e == cudaSuccess) e = upload_slots_adjoint(scenes, slots, n, primes, prime_sums, stream);
+cudaError_t upload_constants(const DeviceScene* scenes, const uint32_t* slots, uint32_t n,
+                             cudaStream_t stream) {
+  cudaError_t e = upload_slots_here(scenes, slots, n, stream);
+  if (e == cudaSuccess) e = upload_slots_media(scenes, slots, n, stream);
+  if (e == cudaSuccess) e = upload_slots_adjoint(scenes, slots, n, stream);
   return e;
 }
 

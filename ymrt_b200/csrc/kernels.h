@@ -129,10 +129,9 @@ static_assert(offsetof(WaveCounters, tracking_caps) == offsetof(WaveCounters, er
               "the tracking functions count through errors + 1");
 
 // Uploads scenes[k] into constant-memory slot slots[k] (k < n; slots ==
-// nullptr: slot k) and the prime tables, in every translation unit that holds
+// nullptr: slot k), in every translation unit that holds
 // wave kernels (each has its own copy of the table).
-cudaError_t upload_constants(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, const uint32_t* primes,
-                             const uint32_t* prime_sums, cudaStream_t stream);
+cudaError_t upload_constants(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, cudaStream_t stream);
 constexpr uint32_t kMaxSceneSlots = 64;
 
 
@@ -236,10 +235,8 @@ void launch_media_extend(uint32_t features, const WaveArgs& w);
 void launch_media_shade(uint32_t features, const WaveArgs& w);
 void launch_adjoint_extend_media(const WaveArgs& w, const WaveOptions& opt);
 void launch_adjoint_shade(bool volumes, uint32_t features, const WaveArgs& w, const WaveOptions& opt);
-cudaError_t upload_slots_media(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, const uint32_t* primes,
-                               const uint32_t* prime_sums, cudaStream_t stream);
-cudaError_t upload_slots_adjoint(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, const uint32_t* primes,
-                                 const uint32_t* prime_sums, cudaStream_t stream);
+cudaError_t upload_slots_media(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, cudaStream_t stream);
+cudaError_t upload_slots_adjoint(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, cudaStream_t stream);
 struct BoundRecord;
 cudaError_t read_bound_media(BoundRecord* out, bool clear, cudaStream_t stream);
 cudaError_t read_bound_adjoint(BoundRecord* out, bool clear, cudaStream_t stream);

@@ -43,9 +43,9 @@ void launch_adjoint_shade(bool volumes, uint32_t features, const WaveArgs& w, co
 
 void prepare_adjoint_kernels() { allow_trace_shared(k_extend<true, kFeatAll, true>); }
 
-cudaError_t upload_slots_adjoint(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, const uint32_t* primes,
-                                 const uint32_t* prime_sums, cudaStream_t stream) {
-  return upload_slots_here(scenes, slots, n, primes, prime_sums, stream);
+cudaError_t upload_slots_adjoint(const DeviceScene* scenes, const uint32_t* slots, uint32_t n,
+                                 cudaStream_t stream) {
+  return upload_slots_here(scenes, slots, n, stream);
 }
 
 cudaError_t read_bound_adjoint(BoundRecord* out, bool clear, cudaStream_t stream) {

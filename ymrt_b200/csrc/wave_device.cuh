@@ -1278,9 +1278,9 @@ static void allow_trace_shared(K kernel) {
 }
 
 // Writes scenes[k] into this translation unit's constant slot slots[k]
-// (k < n; slots == nullptr: slot k) and the prime tables.
+// (k < n; slots == nullptr: slot k).
 static cudaError_t upload_slots_here(const DeviceScene* scenes, const uint32_t* slots, uint32_t n,
-                                     const uint32_t* primes, const uint32_t* prime_sums, cudaStream_t stream) {
+                                     cudaStream_t stream) {
   if (n > (uint32_t)kMaxBatchScenes) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
   uint32_t k = 0;
@@ -1294,11 +1294,6 @@ static cudaError_t upload_slots_here(const DeviceScene* scenes, const uint32_t* 
                                 cudaMemcpyHostToDevice, stream);
     k += run;
   }
-  if (e == cudaSuccess)
-    e = cudaMemcpyToSymbolAsync(c_primes, primes, sizeof(uint32_t) * kHaltonDims, 0, cudaMemcpyHostToDevice, stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyToSymbolAsync(c_prime_sums, prime_sums, sizeof(uint32_t) * kHaltonDims, 0, cudaMemcpyHostToDevice,
-                                stream);
   return e;
 }
 

@@ -52,9 +52,9 @@ void prepare_media_kernels() {
   allow_trace_shared(k_extend<true, kAllNodes | kFeatSpheres>);
 }
 
-cudaError_t upload_slots_media(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, const uint32_t* primes,
-                               const uint32_t* prime_sums, cudaStream_t stream) {
-  return upload_slots_here(scenes, slots, n, primes, prime_sums, stream);
+cudaError_t upload_slots_media(const DeviceScene* scenes, const uint32_t* slots, uint32_t n,
+                               cudaStream_t stream) {
+  return upload_slots_here(scenes, slots, n, stream);
 }
 
 cudaError_t read_bound_media(BoundRecord* out, bool clear, cudaStream_t stream) {

@@ -25,6 +25,7 @@ constexpr int kMaxRayDepth = 64;              // MAX_RAY_DEPTH, src/SceneDefines
 constexpr int kTileRes = 16;                  // TILE_X_RES / TILE_Y_RES
 constexpr int kTilePixels = 256;
 constexpr int kHaltonDims = 1000;             // PRIME_TABLE_SIZE, src/RandomSampler.cuh:12
+constexpr size_t kHaltonTableSize = 3682913;  // sum of the first kHaltonDims primes
 constexpr int kMaxFreePath = 2048;            // MAX_FREE_PATH_LENGTH, src/VolumeEval.cuh:16
 
 enum MaterialType : uint32_t { kDefaultMtl = 0, kLightMtl = 1 };
