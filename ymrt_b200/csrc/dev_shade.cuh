@@ -228,11 +228,6 @@ __device__ __forceinline__ float ggx_lambda(vec3 w, float ax, float ay) {
   if (fabsf(w.z) < 1E-8f) return 0.0f;
   return (-1.0f + sqrtf(1.0f + (sqr(w.x * ax) + sqr(w.y * ay)) / sqr(w.z))) * 0.5f;
 }
-__device__ __forceinline__ float ggx_g1(vec3 w, float ax, float ay) { return 1.0f / (1.0f + ggx_lambda(w, ax, ay)); }
-__device__ __forceinline__ float ggx_g2(vec3 wo, vec3 wi, float ax, float ay) {
-  return 1.0f / (1.0f + ggx_lambda(wo, ax, ay) + ggx_lambda(wi, ax, ay));
-}
-
 // SampleWh: visible-normal sampling (src/BSDF.cuh:158-176). The blend
 // weight and the hemisphere-projection term are evaluated in double, as the
 // reference's double literals make them.
@@ -280,70 +275,67 @@ struct LayeredBsdf {
   __device__ __forceinline__ vec3 to_world(vec3 v) const { return v.x * t + v.y * b + v.z * n; }
 };
 
+// The terms of a microfacet lobe that its evaluation and its sampling share,
+// at half vector wh: the distribution, the masking of wo (g1) and of both
+// directions (g2, summed in the order the reference's call has its two
+// arguments), the Fresnel factor, the half-vector Jacobian of a transmission
+// and the pdf (src/BSDF.cuh:230-255, 300-334).
+struct MicroTerms {
+  float D, g1, g2, dwh, pdf;
+  vec3 fr;
+};
+__device__ __forceinline__ void microfacet_terms(const Lobe& L, vec3 wo, vec3 wi, vec3 wh, bool wi_first,
+                                                     MicroTerms* m) {
+  const float D = ggx_d(wh, L.ax, L.ay);
+  const float lo = ggx_lambda(wo, L.ax, L.ay), li = ggx_lambda(wi, L.ax, L.ay);
+  const float G1 = 1.0f / (1.0f + lo);
+  m->D = D;
+  m->g1 = G1;
+  m->g2 = 1.0f / (1.0f + (wi_first ? li : lo) + (wi_first ? lo : li));
+  const float ni = L.ni, nt = L.nt.x;
+  const float i_ni = safe_rcp(ni);
+  const float c = gmax(dot(wo, wh), 0.0f);
+  if (L.is_metal) m->fr = fresnel_conductor(L.nt * i_ni, L.kt * i_ni, c);
+  else m->fr = vec3(fresnel_dielectric(nt * i_ni, c));
+  if (L.type == kReflect) {
+    m->pdf = D * G1 * 0.25f / gmax(wo.z, 1E-8f);
+  } else {
+    m->dwh = sqr(nt) * fabsf(dot(wi, wh)) / gmax(sqr(ni * dot(wo, wh) + nt * dot(wi, wh)), 1E-12f);
+    m->pdf = D * G1 * fabsf(dot(wo, wh)) * m->dwh / gmax(fabsf(wo.z), 1E-8f);
+  }
+}
+
 // Lambert / MicrofacetReflection / MicrofacetTransmission ::Eval (src/BSDF.cuh:185-375).
-// lobe_eval and lobe_sample are out of line: the layered BSDF's evaluation
-// and sampling call them from several sites, and one copy of each keeps the
-// shading kernels' instruction footprint small (A/B on one B200: textured
-// 1280x720 32-spp frame 742 -> 717 ms, the instanced 1080p 64-spp bench frame
-// 216.5 -> 215.3 ms, volumetric unchanged; lobe_eval alone out of line cost
-// the bench frame 1.3%).
+// lobe_eval and lobe_sample are out of line: the layered BSDF calls them from
+// several sites, and one copy of each keeps the shading kernels' instruction
+// footprint small.
 static __device__ __noinline__ vec3 lobe_eval(const Lobe& L, vec3 wo, vec3 wi, float* pdf) {
+  *pdf = 0.0f;
+  const bool same = same_hemisphere(wo, wi);
   if (L.type == kLambert) {
-    if (!same_hemisphere(wo, wi)) {
-      *pdf = 0.0f;
-      return vec3(0.0f);
-    }
+    if (!same) return vec3(0.0f);
     const float c = gmax(wi.z, 0.0f);
     *pdf = c * kInvPi;
     return L.albedo * c * kInvPi;
   }
-  if (L.type == kReflect) {
-    if (!same_hemisphere(wo, wi) || wo.z < 0.f || wi.z < 0.f) {
-      *pdf = 0.0f;
-      return vec3(0.0f);
-    }
-    vec3 wh = wi + wo;
-    const float len = length(wh);
-    if (fabsf(len) < 1E-8f) {
-      *pdf = 0.0f;
-      return vec3(0.0f);
-    }
-    wh /= len;
-    const float D = ggx_d(wh, L.ax, L.ay);
-    const float G1 = ggx_g1(wo, L.ax, L.ay);
-    const float G2 = ggx_g2(wo, wi, L.ax, L.ay);
-    const float i_ni = safe_rcp(L.ni);
-    const float c = gmax(dot(wo, wh), 0.0f);
-    const vec3 fr = L.is_metal ? fresnel_conductor(L.nt * i_ni, L.kt * i_ni, c) : vec3(fresnel_dielectric(L.nt.x * i_ni, c));
-    *pdf = D * G1 * 0.25f / gmax(wo.z, 1E-8f);
-    return L.albedo * D * G2 * 0.25f * fr / gmax(wo.z, 1E-8f);
-  }
-  // transmission
   const float ni = L.ni, nt = L.nt.x;
-  if (same_hemisphere(wo, wi)) {
-    *pdf = 0.0f;
-    return vec3(0.0f);
-  }
-  vec3 wh = -(ni * wo + nt * wi);
-  if (!same_hemisphere(wo, wh)) {
-    *pdf = 0.0f;
-    return vec3(0.0f);
+  vec3 wh;
+  if (L.type == kReflect) {
+    if (!same || wo.z < 0.f || wi.z < 0.f) return vec3(0.0f);
+    wh = wi + wo;
+  } else {
+    if (same) return vec3(0.0f);
+    wh = -(ni * wo + nt * wi);
+    if (!same_hemisphere(wo, wh)) return vec3(0.0f);
   }
   const float len = length(wh);
-  if (fabsf(len) < 1E-8f) {
-    *pdf = 0.0f;
-    return vec3(0.0f);
-  }
+  if (fabsf(len) < 1E-8f) return vec3(0.0f);
   wh /= len;
-  const float D = ggx_d(wh, L.ax, L.ay);
-  const float G1 = ggx_g1(wo, L.ax, L.ay);
-  const float G2 = ggx_g2(wo, wi, L.ax, L.ay);
-  const float dwh = sqr(nt) * fabsf(dot(wi, wh)) / gmax(sqr(ni * dot(wo, wh) + nt * dot(wi, wh)), 1E-12f);
-  const float i_ni = safe_rcp(ni);
-  const float c = gmax(dot(wo, wh), 0.0f);
-  const float fr = fresnel_dielectric(nt * i_ni, c);
-  *pdf = D * G1 * fabsf(dot(wo, wh)) * dwh / gmax(fabsf(wo.z), 1E-8f);
-  return L.albedo * (1.0f - fr) * fabsf(dot(wo, wh) / gmax(fabsf(wo.z), 1E-8f)) * G2 * D * dwh * sqr(ni / nt);
+  MicroTerms m;
+  microfacet_terms(L, wo, wi, wh, false, &m);
+  *pdf = m.pdf;
+  if (L.type == kReflect) return L.albedo * m.D * m.g2 * 0.25f * m.fr / gmax(wo.z, 1E-8f);
+  return L.albedo * (1.0f - m.fr.x) * fabsf(dot(wo, wh) / gmax(fabsf(wo.z), 1E-8f)) * m.g2 * m.D * m.dwh * sqr(ni / nt);
 }
 
 // ::Sample of the three lobe types (src/BSDF.cuh:205-213, 258-283, 336-374).
@@ -362,31 +354,16 @@ static __device__ __noinline__ bool lobe_sample(const Lobe& L, float u0, float u
   }
   const vec3 wh = sample_wh(wo, u0, u1, L.ax, L.ay);
   if (!same_hemisphere(wo, wh) || dot(wo, wh) < 0.0f) return false;
-  if (L.type == kReflect) {
-    *wi = reflect(wo, wh);
-    if (!same_hemisphere(*wi, wo)) return false;
-    const float D = ggx_d(wh, L.ax, L.ay);
-    const float G1 = ggx_g1(wo, L.ax, L.ay);
-    const float G2 = ggx_g2(wo, *wi, L.ax, L.ay);
-    const float i_ni = safe_rcp(L.ni);
-    const float c = gmax(dot(wo, wh), 0.0f);
-    const vec3 fr = L.is_metal ? fresnel_conductor(L.nt * i_ni, L.kt * i_ni, c) : vec3(fresnel_dielectric(L.nt.x * i_ni, c));
-    *pdf = D * G1 * 0.25f / gmax(wo.z, 1E-8f);
-    *weight = L.albedo * G2 * fr / G1;
-    return true;
-  }
+  const bool mirror = L.type == kReflect;
   const float ni = L.ni, nt = L.nt.x;
-  if (!refract(wo, wh, ni, nt, wi)) return false;
-  if (same_hemisphere(*wi, wo)) return false;
-  const float D = ggx_d(wh, L.ax, L.ay);
-  const float G1 = ggx_g1(wo, L.ax, L.ay);
-  const float G2 = ggx_g2(*wi, wo, L.ax, L.ay);
-  const float dwh = sqr(nt) * fabsf(dot(*wi, wh)) / gmax(sqr(ni * dot(wo, wh) + nt * dot(*wi, wh)), 1E-12f);
-  const float i_ni = safe_rcp(ni);
-  const float c = gmax(dot(wo, wh), 0.0f);
-  const float fr = fresnel_dielectric(nt * i_ni, c);
-  *pdf = D * G1 * fabsf(dot(wo, wh)) * dwh / gmax(fabsf(wo.z), 1E-8f);
-  *weight = L.albedo * (1.0f - fr) * sqr(ni / nt) * G2 / G1;
+  if (mirror) *wi = reflect(wo, wh);
+  else if (!refract(wo, wh, ni, nt, wi)) return false;
+  if (same_hemisphere(*wi, wo) != mirror) return false;
+  MicroTerms m;
+  microfacet_terms(L, wo, *wi, wh, !mirror, &m);
+  *pdf = m.pdf;
+  if (mirror) *weight = L.albedo * m.g2 * m.fr / m.g1;
+  else *weight = L.albedo * (1.0f - m.fr.x) * sqr(ni / nt) * m.g2 / m.g1;
   return true;
 }
 
@@ -954,15 +931,18 @@ __device__ __forceinline__ vec3 background(vec3 d) {
 }
 
 // indirect_light_clamp (src/Shading.cu:61-81).
-__device__ __forceinline__ vec3 indirect_clamp(const RenderSetting& rs, vec3 c, int depth) {
-  if (!(rs.enable_indirect_clamp && depth > 1)) return c;
-  if (!(rs.indirect_limit > 0.0f)) return vec3(0.0f);
+// The clamp itself, with its two powers, is out of line: most renders never
+// run it.
+static __device__ __noinline__ vec3 clamp_to_limit(vec3 c, float limit) {
+  if (!(limit > 0.0f)) return vec3(0.0f);
   const float lum = luminance(c);
   if (lum <= 1E-10f) return c;
-  const float limit = rs.indirect_limit;
   const float pw = gmin(0.05f + 0.25f * (powf(lum / limit, 1.5f)), 1.0f);
   const float sf = powf(limit / (limit + lum), pw);
   return c * sf;
+}
+__device__ __forceinline__ vec3 indirect_clamp(const RenderSetting& rs, vec3 c, int depth) {
+  return rs.enable_indirect_clamp && depth > 1 ? clamp_to_limit(c, rs.indirect_limit) : c;
 }
 
 }  // namespace ym

@@ -658,13 +658,8 @@ void launch_extend_surface(const WaveArgs& w) {
 template <uint32_t kF>
 void launch_shade_surface(const ShadowQueue* defer, const WaveArgs& w) {
   constexpr uint32_t kS = surface_features(kF);
-  const ShadowQueue none{};
-  if (defer)
-    k_shade<false, true, false, kS><<<w.blocks, kTraceBlock, 0, w.stream>>>(w.A, w.ctl, w.H, w.B, w.jobs, w.counters,
-                                                                            *defer);
-  else
-    k_shade<false, false, false, kS><<<w.blocks, kTraceBlock, 0, w.stream>>>(w.A, w.ctl, w.H, w.B, w.jobs,
-                                                                             w.counters, none);
+  if (defer) launch_shade<false, true, false, kS>(w, *defer);
+  else launch_shade<false, false, false, kS>(w, ShadowQueue{});
 }
 
 }  // namespace
@@ -687,6 +682,10 @@ void prepare_persistent_grids() {
   }
   allow_trace_shared(k_extend<false, 0>);
   allow_trace_shared(k_extend<false, kFeatSpheres>);
+  allow_shade_shared<false, false, 0>();
+  allow_shade_shared<false, false, kFeatSpheres>();
+  allow_shade_shared<false, false, kFeatTextures>();
+  allow_shade_shared<false, false, kFeatSpheres | kFeatTextures>();
   prepare_media_kernels();
   prepare_adjoint_kernels();
   g_grids = g;

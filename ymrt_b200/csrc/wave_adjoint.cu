@@ -12,9 +12,7 @@ namespace {
 
 template <uint32_t kS>
 void surface_adjoint_shade(const WaveArgs& w, const WaveOptions& opt) {
-  const ShadowQueue none{};
-  k_shade<false, false, true, kS><<<w.blocks, kTraceBlock, 0, w.stream>>>(w.A, w.ctl, w.H, w.B, w.jobs, w.counters,
-                                                                          none, opt.grads, opt.grad_materials);
+  launch_shade<false, false, true, kS>(w, ShadowQueue{}, opt.grads, opt.grad_materials);
 }
 
 }  // namespace
@@ -28,9 +26,8 @@ void launch_adjoint_extend_media(const WaveArgs& w, const WaveOptions& opt) {
 
 void launch_adjoint_shade(bool volumes, uint32_t features, const WaveArgs& w, const WaveOptions& opt) {
   if (volumes) {
-    const ShadowQueue none{};
-    k_shade<true, false, true, kFeatAll><<<w.blocks, kTraceBlock, 0, w.stream>>>(
-        w.A, w.ctl, w.H, w.B, w.jobs, w.counters, none, opt.grads, opt.grad_materials, opt.grid_grads, opt.grid_tex);
+    launch_shade<true, false, true, kFeatAll>(w, ShadowQueue{}, opt.grads, opt.grad_materials, opt.grid_grads,
+                                              opt.grid_tex);
     return;
   }
   switch (surface_features(features)) {
@@ -41,7 +38,14 @@ void launch_adjoint_shade(bool volumes, uint32_t features, const WaveArgs& w, co
   }
 }
 
-void prepare_adjoint_kernels() { allow_trace_shared(k_extend<true, kFeatAll, true>); }
+void prepare_adjoint_kernels() {
+  allow_trace_shared(k_extend<true, kFeatAll, true>);
+  allow_shade_shared<false, true, 0>();
+  allow_shade_shared<false, true, kFeatSpheres>();
+  allow_shade_shared<false, true, kFeatTextures>();
+  allow_shade_shared<false, true, kFeatSpheres | kFeatTextures>();
+  allow_shade_shared<true, true, kFeatAll>();
+}
 
 cudaError_t upload_slots_adjoint(const DeviceScene* scenes, const uint32_t* slots, uint32_t n,
                                  cudaStream_t stream) {

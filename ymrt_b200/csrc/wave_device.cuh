@@ -369,11 +369,8 @@ __device__ __noinline__ vec3 trace_tr(uint32_t scene, TraversalStack& st, vec3 o
     }
     ClosestHit ch;
     const bool hit = trace_closest_impl<(kF & kFeatSpheres) != 0>(scene, st, o, d, ray_t, last_inst, last_tri, true, &ch, tests, nodes);
-    if (!hit) {
-      tr *= eval_tr<kF, kAdj>(S, o, d, rt, gmax(max_d - traced, 0.0f), hs, errors, am);
-      break;
-    }
-    tr *= eval_tr<kF, kAdj>(S, o, d, rt, ch.t, hs, errors, am);
+    tr *= eval_tr<kF, kAdj>(S, o, d, rt, hit ? ch.t : gmax(max_d - traced, 0.0f), hs, errors, am);
+    if (!hit) break;
     traced += ch.t;
     vec3 hp, herr, hng;
     fetch_geometry_normal<kF>(S, ch.inst, ch.tri, vec3(ch.b0, ch.b1, ch.b2), &hp, &herr, &hng);
@@ -386,6 +383,13 @@ __device__ __noinline__ vec3 trace_tr(uint32_t scene, TraversalStack& st, vec3 o
   }
   return tr;
 }
+
+// A direction toward a light: radiance and pdf, and (shape lights) the point
+// reached on it with its error and geometric normal.
+struct LightSample {
+  vec3 dir, pos, err, ng, Li;
+  float pdf;
+};
 
 // DistantLight::SampleLi / EvalLi (src/Light.h:343-386).
 __device__ __forceinline__ void distant_sample_li(const DeviceScene& S, const DistantLight& L, float u0, float u1, vec3* wi,
@@ -418,29 +422,6 @@ __device__ __forceinline__ vec3 distant_eval_li(const DeviceScene& S, const Dist
   return L.light_color * L.intensity * (*pdf);
 }
 
-// Shading-point context the light estimators share.
-struct SurfaceNee {
-  vec3 ray_dir, p, p_err, ng;
-  uint32_t inst, tri;
-  const RayTransfer* rt;
-  const NearbyHit* nb;
-  int n_nb;
-  bool media;  // the render's enable_volume_scattering
-  uint32_t slot;  // scene slot
-};
-
-// Transmittance of an unoccluded surface shadow ray (the volume part of the
-// reference's EvalShapeLight / EvalDistantLight).
-template <bool kVol, uint32_t kF, bool kAdj = false>
-__device__ __forceinline__ vec3 surface_shadow_tr(const DeviceScene& S, TraversalStack& st, const SurfaceNee& c, vec3 so,
-                                                  vec3 ldir, float maxd, bool tb, PathSampler& hs, uint32_t* errors,
-                                                  uint32_t* tests, uint32_t* nodes, const MediumAdj* am = nullptr) {
-  if (!kVol || !c.media) return vec3(1.0f);
-  RayTransfer srt = *c.rt;
-  if (tb) boundary_transition(S, srt, c.nb, c.n_nb, errors);
-  return trace_tr<kF, kAdj>(c.slot, st, so, normalize(ldir), maxd, c.inst, c.tri, srt, hs, errors, tests, nodes, am);
-}
-
 // ------------------------------------------------- path-replay adjoint ---
 //
 // Gradients of an image loss with respect to each material's diffuse albedo
@@ -461,8 +442,6 @@ constexpr float kParamStep = 1e-3f;       // central-difference step of df/dp
 struct AdjCtx {
   vec3 weight;                            // dLoss/dI (per path) * throughput: the weight of this vertex's NEE
   float g[kGradParams];                   // accumulated dLoss/dp
-  float* grid_grads;                      // dLoss/d(density-grid value), or null
-  uint32_t grid_tex;                      // the differentiated grid node
   // Per-lobe derivative data of the vertex's layered BSDF (channel-diagonal
   // in albedo: each channel's albedo moves only that channel of f):
   vec3 lambert_coeff;                     // the diffuse lobe's colour per unit albedo
@@ -567,294 +546,45 @@ __device__ __forceinline__ void emit_shadow_ray(const ShadowEmit& em, vec3 o, ve
   em.q.path[slot] = em.path;
 }
 
-// One next-event shadow ray of a surface vertex toward a light, with MIS
-// weight `mis`, clamped BSDF value fc and radiance Lc; the light-selection
-// pdf enters as (x * mul) / div, the form each estimator uses. Traced here
-// (direct += its unoccluded contribution, times the media transmittance)
-// or, with kDefer, queued for k_connect.
-template <bool kVol, bool kDefer, uint32_t kF>
-__device__ __forceinline__ void nee_shadow_ray(const DeviceScene& S, TraversalStack& st, const SurfaceNee& c,
-                                               const ShadowEmit& em, vec3 so, vec3 ldir, float maxd, bool tb,
-                                               float mis, vec3 fc, vec3 Lc, float mul, float div, vec3* direct,
-                                               PathSampler& hs, uint32_t* shadow_rays, uint32_t* tests,
-                                               uint32_t* nodes, uint32_t* errors, AdjCtx* adj = nullptr,
-                                               const LayeredBsdf* B = nullptr) {
-  ++*shadow_rays;
-  if (kDefer) {
-    emit_shadow_ray(em, so, normalize(ldir), maxd, ((mis * vec3(1.0f) * fc * Lc) * mul) / div);
+// A light chosen for next-event estimation: a shape light (triangle or
+// sphere) or a distant light, and the probability of the choice.
+struct ChosenLight {
+  bool distant;
+  int index;        // distant: into S.distant_lights
+  float area;       // shape lights
+  float select_pdf;
+  LightTri tri;     // shape lights
+};
+template <uint32_t kF>
+__device__ __forceinline__ void choose_light(const DeviceScene& S, bool distant, PathSampler& hs, ChosenLight& L) {
+  L.distant = distant;
+  const float u = sample1d(hs, S);
+  if (distant) {
+    L.select_pdf = 1.0f / float(S.distant_light_count);
+    L.index = gmax(gmin((int)(u * S.distant_light_count), (int)S.distant_light_count - 1), 0);
     return;
   }
-  if (!trace_occluded_impl<(kF & kFeatSpheres) != 0>(c.slot, st, so, normalize(ldir), maxd, tests, nodes)) {
-    const PathSampler hs0 = hs;
-    const vec3 tr = surface_shadow_tr<kVol, kF>(S, st, c, so, ldir, maxd, tb, hs, errors, tests, nodes);
-    *direct += mis * tr * fc * Lc;
-    if constexpr (kVol) {
-      if (adj && adj->grid_grads && c.media) {
-        // the transmittance's density-grid terms: replay its tracking with the
-        // same samples, weighted by this ray's share of dLoss
-        const MediumAdj am{adj->weight * (mul / div) * (mis * tr * fc * Lc), adj->grid_tex, adj->grid_grads};
-        if (max_component(vabs(am.scale)) > 0.0f) {
-          PathSampler h2 = hs0;
-          surface_shadow_tr<kVol, kF, true>(S, st, c, so, ldir, maxd, tb, h2, errors, tests, nodes, &am);
-        }
-      }
-    }
-    if (adj) {
-      // d(direct)/dp = mis * tr * fc * (df/dp)/f * Lc, scaled like the estimator
-      const vec3 wo = B->to_local(-c.ray_dir), wi = B->to_local(ldir);
-      add_relative_grads(adj, *B, wo, wi, adj->weight * (mul / div), mis * tr * fc * Lc);
-    }
-  }
+  const ShapeLight sl = S.shape_lights[sample_light_power(S, u, &L.select_pdf)];
+  L.area = sl.area;
+  L.tri = load_light_tri<kF>(S, sl);
 }
-
-// EvalShapeLight (src/Shading.cu:294-417).
-template <bool kVol, bool kDefer, uint32_t kF>
-__device__ __forceinline__ vec3 eval_shape_light(const DeviceScene& S, TraversalStack& st, const LayeredBsdf& B,
-                                                 const SurfaceNee& c, const ShadowEmit& em, PathSampler& hs,
-                                                 uint32_t* shadow_rays, uint32_t* tests, uint32_t* nodes,
-                                                 uint32_t* errors, AdjCtx* adj = nullptr) {
-  if (S.shape_light_count == 0) return vec3(0.0f);
-  vec3 direct(0.0f);
-  const vec3 wo = B.to_local(-c.ray_dir);
-  float select_pdf = 0.0f;
-  const int li = sample_light_power(S, sample1d(hs, S), &select_pdf);
-  const ShapeLight L = S.shape_lights[li];
-  const LightTri lt = load_light_tri<kF>(S, L);
-  {
-    float u0, u1;
-    sample2d(hs, S, &u0, &u1);
-    vec3 ldir(0.0f), lpos(0.0f), lerr(0.0f), lng(0.0f), Li(0.0f);
-    float lpdf = 0.0f;
-    const bool valid = light_sample_li<kF>(lt, L.area, c.p, u0, u1, &ldir, &lpos, &lerr, &lng, &Li, &lpdf);
-    const vec3 lwi = B.to_local(ldir);
-    float wpdf = 0.0f;
-    const vec3 f = bsdf_eval(B, wo, lwi, &wpdf);
-    if (max_component(f) > kMinColorEps && valid) {
-      const vec3 so = offset_ray_origin(c.p, c.p_err, ldir, c.ng);
-      const float maxd = length(offset_ray_origin(lpos, lerr, -ldir, lng) - c.p) * kShadowRayClamp;
-      const bool tb = dot(-c.ray_dir, c.ng) * dot(ldir, c.ng) < 0.0f;
-      const bool invalid = (!same_hemisphere(wo, lwi) && !tb) || (same_hemisphere(wo, lwi) && tb);
-      if (!invalid)
-        nee_shadow_ray<kVol, kDefer, kF>(S, st, c, em, so, ldir, maxd, tb, power_heuristic(lpdf, wpdf),
-                                     vmin(f, vec3(kMaxColorClamp)), vmin(Li, vec3(kMaxColorClamp)),
-                                     safe_rcp(select_pdf), 1.0f, &direct, hs, shadow_rays, tests, nodes, errors, adj, &B);
-    }
-  }
-  {
-    float u0, u1, u2;
-    sample3d(hs, S, &u0, &u1, &u2);
-    vec3 bw, bwi;
-    float bpdf = 0.0f;
-    if (bsdf_sample(B, wo, &bw, &bwi, &bpdf, u0, u1, u2)) {
-      const vec3 ldir = B.to_world(bwi);
-      vec3 lpos(0.0f), lerr(0.0f), lng(0.0f);
-      float wpdf = 0.0f;
-      const vec3 Li = light_eval_li<kF>(lt, L.area, c.p, ldir, &lpos, &lerr, &lng, &wpdf);
-      if (max_component(Li) > kMinColorEps) {
-        const vec3 so = offset_ray_origin(c.p, c.p_err, ldir, c.ng);
-        const float maxd = length(offset_ray_origin(lpos, lerr, -ldir, lng) - c.p) * kShadowRayClamp;
-        const bool tb = dot(-c.ray_dir, c.ng) * dot(ldir, c.ng) < 0.0f;
-        const bool invalid = (!same_hemisphere(wo, bwi) && !tb) || (same_hemisphere(wo, bwi) && tb);
-        if (!invalid)
-          nee_shadow_ray<kVol, kDefer, kF>(S, st, c, em, so, ldir, maxd, tb, power_heuristic(bpdf, wpdf),
-                                       vmin(bw, vec3(kMaxColorClamp)), vmin(Li, vec3(kMaxColorClamp)),
-                                       safe_rcp(select_pdf), 1.0f, &direct, hs, shadow_rays, tests, nodes, errors, adj, &B);
-      }
-    }
-  }
-  return direct * safe_rcp(select_pdf);
-}
-
-// EvalDistantLight (src/Shading.cu:83-198).
-template <bool kVol, bool kDefer, uint32_t kF>
-__device__ __forceinline__ vec3 eval_distant_light(const DeviceScene& S, TraversalStack& st, const LayeredBsdf& B,
-                                                   const SurfaceNee& c, const ShadowEmit& em, PathSampler& hs,
-                                                   uint32_t* shadow_rays, uint32_t* tests, uint32_t* nodes,
-                                                   uint32_t* errors, AdjCtx* adj = nullptr) {
-  if (S.distant_light_count == 0) return vec3(0.0f);
-  vec3 direct(0.0f);
-  const vec3 wo = B.to_local(-c.ray_dir);
-  const float select_pdf = 1.0f / float(S.distant_light_count);
-  const int li = gmax(gmin((int)(sample1d(hs, S) * S.distant_light_count), (int)S.distant_light_count - 1), 0);
-  const DistantLight L = S.distant_lights[li];
-  {
-    float u0, u1;
-    sample2d(hs, S, &u0, &u1);
-    vec3 ldir(0.0f), Li(0.0f);
-    float lpdf = 0.0f;
-    distant_sample_li(S, L, u0, u1, &ldir, &Li, &lpdf);
-    const vec3 lwi = B.to_local(ldir);
-    float wpdf = 0.0f;
-    const vec3 f = bsdf_eval(B, wo, lwi, &wpdf);
-    if (max_component(f) > kMinColorEps) {
-      const vec3 so = offset_ray_origin(c.p, c.p_err, ldir, c.ng);
-      const bool tb = dot(-c.ray_dir, c.ng) * dot(ldir, c.ng) < 0.0f;
-      const bool invalid = (!same_hemisphere(wo, lwi) && !tb) || (same_hemisphere(wo, lwi) && tb);
-      if (!invalid)
-        nee_shadow_ray<kVol, kDefer, kF>(S, st, c, em, so, ldir, kTMax, tb, power_heuristic(lpdf, wpdf),
-                                     vmin(f, vec3(kMaxColorClamp)), vmin(Li, vec3(kMaxColorClamp)), 1.0f,
-                                     select_pdf, &direct, hs, shadow_rays, tests, nodes, errors, adj, &B);
-    }
-  }
-  {
-    float u0, u1, u2;
-    sample3d(hs, S, &u0, &u1, &u2);
-    vec3 bw, bwi;
-    float bpdf = 0.0f;
-    if (bsdf_sample(B, wo, &bw, &bwi, &bpdf, u0, u1, u2)) {
-      const vec3 ldir = B.to_world(bwi);
-      float wpdf = 0.0f;
-      const vec3 Li = distant_eval_li(S, L, ldir, &wpdf);
-      if (max_component(Li) > kMinColorEps) {
-        const vec3 so = offset_ray_origin(c.p, c.p_err, ldir, c.ng);
-        const bool tb = dot(-c.ray_dir, c.ng) * dot(ldir, c.ng) < 0.0f;
-        const bool invalid = (!same_hemisphere(wo, bwi) && !tb) || (same_hemisphere(wo, bwi) && tb);
-        if (!invalid)
-          nee_shadow_ray<kVol, kDefer, kF>(S, st, c, em, so, ldir, kTMax, tb, power_heuristic(bpdf, wpdf),
-                                       vmin(bw, vec3(kMaxColorClamp)), vmin(Li, vec3(kMaxColorClamp)), 1.0f,
-                                       select_pdf, &direct, hs, shadow_rays, tests, nodes, errors, adj, &B);
-      }
-    }
-  }
-  return direct / select_pdf;
-}
-
-// Density-grid terms of one volume shadow ray's transmittance (the adjoint
-// pass): its tracking replayed from the sampler state `hs` it started from,
-// weighted by av->scale (dLoss/dI times throughput) times the ray's
-// contribution to the estimate (contrib / select_pdf).
+// A direction toward the light from `p` (false: none), its radiance and pdf;
+// shape lights also give the point on the light with its error and normal.
 template <uint32_t kF>
-__device__ __noinline__ void volume_shadow_grad(uint32_t slot, TraversalStack& st, vec3 pos, vec3 dir, float maxd,
-                                                const RayTransfer& rt, PathSampler hs, vec3 contrib, float select_pdf,
-                                                const MediumAdj* av, uint32_t* errors, uint32_t* tests,
-                                                uint32_t* nodes) {
-  if (!av || !av->grads || !(select_pdf > 0.0f)) return;
-  const MediumAdj am{av->scale * contrib / select_pdf, av->grid_tex, av->grads};
-  if (!(max_component(vabs(am.scale)) > 0.0f)) return;
-  RayTransfer srt = rt;
-  trace_tr<kF, true>(slot, st, pos, dir, maxd, kEmpty, kEmpty, srt, hs, errors, tests, nodes, &am);
+__device__ __forceinline__ bool sample_chosen_light(const DeviceScene& S, const ChosenLight& L, vec3 p, float u0, float u1,
+                                                 LightSample& q) {
+  if (L.distant) {
+    distant_sample_li(S, S.distant_lights[L.index], u0, u1, &q.dir, &q.Li, &q.pdf);
+    return true;
+  }
+  return light_sample_li<kF>(L.tri, L.area, p, u0, u1, &q.dir, &q.pos, &q.err, &q.ng, &q.Li, &q.pdf);
 }
-
-// EvalVolumeShapeLight / EvalVolumeDistantLight (src/Shading.cu:202-291, 419-513):
-// next-event estimation at a scattering point inside the media. kAdj: the
-// adjoint pass, which also adds each shadow ray's density-grid terms (av).
-template <uint32_t kF, bool kAdj = false>
-__device__ __noinline__ vec3 eval_volume_lights(uint32_t slot, TraversalStack& st, bool distant, int n,
-                                                const float* gs, const float* vw, vec3 ray_dir, const RayTransfer& rt,
-                                                vec3 pos, PathSampler& hs, uint32_t* shadow_rays, uint32_t* tests,
-                                                uint32_t* nodes, uint32_t* errors, const MediumAdj* av = nullptr) {
-  const DeviceScene& S = c_scenes[slot];
-  vec3 direct(0.0f);
-  if (distant) {
-    if (S.distant_light_count == 0 || n == 0) return vec3(0.0f);
-    const float select_pdf = 1.0f / float(S.distant_light_count);
-    const int li = gmax(gmin((int)(sample1d(hs, S) * S.distant_light_count), (int)S.distant_light_count - 1), 0);
-    const DistantLight L = S.distant_lights[li];
-    {
-      float u0, u1;
-      sample2d(hs, S, &u0, &u1);
-      vec3 ldir(0.0f), Li(0.0f);
-      float lpdf = 0.0f;
-      distant_sample_li(S, L, u0, u1, &ldir, &Li, &lpdf);
-      float wpdf = 0.0f;
-      const float pw = eval_mixed_phases(vw, gs, n, -ray_dir, ldir, &wpdf);
-      if (pw > kMinColorEps) {
-        ++*shadow_rays;
-        if (!trace_occluded_impl<(kF & kFeatSpheres) != 0>(slot, st, pos, normalize(ldir), kTMax, tests, nodes)) {
-          RayTransfer srt = rt;
-          const PathSampler hs0 = hs;
-          const vec3 tr = trace_tr<kF>(slot, st, pos, normalize(ldir), kTMax, kEmpty, kEmpty, srt, hs, errors, tests, nodes);
-          const float mis = power_heuristic(lpdf, wpdf);
-          const vec3 contrib = mis * tr * gmin(pw, kMaxColorClamp) * vmin(Li, vec3(kMaxColorClamp));
-          direct += contrib;
-          if constexpr (kAdj)
-            volume_shadow_grad<kF>(slot, st, pos, normalize(ldir), kTMax, rt, hs0, contrib, select_pdf, av, errors,
-                                   tests, nodes);
-        }
-      }
-    }
-    {
-      float u0, u1;
-      sample2d(hs, S, &u0, &u1);
-      vec3 pwi;
-      float pspdf = 0.0f, pw = 0.0f;
-      if (sample_mixed_phases(vw, gs, n, u0, u1, -ray_dir, &pw, &pwi, &pspdf)) {
-        float wpdf = 0.0f;
-        const vec3 Li = distant_eval_li(S, L, pwi, &wpdf);
-        if (max_component(Li) > kMinColorEps) {
-          ++*shadow_rays;
-          if (!trace_occluded_impl<(kF & kFeatSpheres) != 0>(slot, st, pos, normalize(pwi), kTMax, tests, nodes)) {
-            RayTransfer srt = rt;
-            const PathSampler hs0 = hs;
-            const vec3 tr = trace_tr<kF>(slot, st, pos, normalize(pwi), kTMax, kEmpty, kEmpty, srt, hs, errors, tests, nodes);
-            const float mis = power_heuristic(pspdf, wpdf);
-            const vec3 contrib = mis * tr * gmin(pw, kMaxColorClamp) * vmin(Li, vec3(kMaxColorClamp));
-            direct += contrib;
-            if constexpr (kAdj)
-              volume_shadow_grad<kF>(slot, st, pos, normalize(pwi), kTMax, rt, hs0, contrib, select_pdf, av, errors,
-                                     tests, nodes);
-          }
-        }
-      }
-    }
-    return direct / select_pdf;
-  }
-  if (S.shape_light_count == 0 || n == 0) return vec3(0.0f);
-  float select_pdf = 0.0f;
-  const int li = sample_light_power(S, sample1d(hs, S), &select_pdf);
-  const ShapeLight L = S.shape_lights[li];
-  const LightTri lt = load_light_tri<kF>(S, L);
-  {
-    float u0, u1;
-    sample2d(hs, S, &u0, &u1);
-    vec3 ldir(0.0f), lpos(0.0f), lerr(0.0f), lng(0.0f), Li(0.0f);
-    float lpdf = 0.0f;
-    const bool valid = light_sample_li<kF>(lt, L.area, pos, u0, u1, &ldir, &lpos, &lerr, &lng, &Li, &lpdf);
-    float wpdf = 0.0f;
-    const float pw = eval_mixed_phases(vw, gs, n, -ray_dir, ldir, &wpdf);
-    if (pw > kMinColorEps && valid) {
-      const float maxd = length(offset_ray_origin(lpos, lerr, -ldir, lng) - pos) * kShadowRayClamp;
-      ++*shadow_rays;
-      if (!trace_occluded_impl<(kF & kFeatSpheres) != 0>(slot, st, pos, normalize(ldir), maxd, tests, nodes)) {
-        RayTransfer srt = rt;
-        const PathSampler hs0 = hs;
-        const vec3 tr = trace_tr<kF>(slot, st, pos, normalize(ldir), maxd, kEmpty, kEmpty, srt, hs, errors, tests, nodes);
-        const float mis = power_heuristic(lpdf, wpdf);
-        const vec3 contrib = mis * tr * gmin(pw, kMaxColorClamp) * vmin(Li, vec3(kMaxColorClamp));
-        direct += contrib;
-        if constexpr (kAdj)
-          volume_shadow_grad<kF>(slot, st, pos, normalize(ldir), maxd, rt, hs0, contrib, select_pdf, av, errors,
-                                 tests, nodes);
-      }
-    }
-  }
-  {
-    float u0, u1;
-    sample2d(hs, S, &u0, &u1);
-    vec3 pwi;
-    float pspdf = 0.0f, pw = 0.0f;
-    if (sample_mixed_phases(vw, gs, n, u0, u1, -ray_dir, &pw, &pwi, &pspdf)) {
-      vec3 lpos(0.0f), lerr(0.0f), lng(0.0f);
-      float wpdf = 0.0f;
-      const vec3 Li = light_eval_li<kF>(lt, L.area, pos, pwi, &lpos, &lerr, &lng, &wpdf);
-      if (max_component(Li) > kMinColorEps) {
-        const float maxd = length(offset_ray_origin(lpos, lerr, -pwi, lng) - pos) * kShadowRayClamp;
-        ++*shadow_rays;
-        if (!trace_occluded_impl<(kF & kFeatSpheres) != 0>(slot, st, pos, normalize(pwi), maxd, tests, nodes)) {
-          RayTransfer srt = rt;
-          const PathSampler hs0 = hs;
-          const vec3 tr = trace_tr<kF>(slot, st, pos, normalize(pwi), maxd, kEmpty, kEmpty, srt, hs, errors, tests, nodes);
-          const float mis = power_heuristic(pspdf, wpdf);
-          const vec3 contrib = mis * tr * gmin(pw, kMaxColorClamp) * vmin(Li, vec3(kMaxColorClamp));
-          direct += contrib;
-          if constexpr (kAdj)
-            volume_shadow_grad<kF>(slot, st, pos, normalize(pwi), maxd, rt, hs0, contrib, select_pdf, av, errors,
-                                   tests, nodes);
-        }
-      }
-    }
-  }
-  return select_pdf > 0.0f ? (direct / select_pdf) : vec3(0.0f);
+// The light's radiance along a direction from `p` (zero: not hit) and the pdf
+// sample_chosen_light would give it.
+template <uint32_t kF>
+__device__ __forceinline__ void eval_chosen_light(const DeviceScene& S, const ChosenLight& L, vec3 p, LightSample& q) {
+  q.Li = L.distant ? distant_eval_li(S, S.distant_lights[L.index], q.dir, &q.pdf)
+                   : light_eval_li<kF>(L.tri, L.area, p, q.dir, &q.pos, &q.err, &q.ng, &q.pdf);
 }
 
 // kDefer (surfaces only, no indirect clamp): next-event shadow rays are queued
@@ -866,31 +596,41 @@ __device__ __noinline__ vec3 eval_volume_lights(uint32_t slot, TraversalStack& s
 // and each material vertex adds its terms of dLoss/dParam (see AdjCtx) to
 // `grads` (per-block sums in shared memory, then one atomic per touched slot).
 //
-// Resident blocks per SM the register allocation is held to (measured on one
-// box, CUDA-event A/B): forward surfaces four (128 registers, a few spills;
-// the 1080p 64-spp bench frame 220.4 -> 217.4 ms against three at 168);
-// forward media without the texture nodes three (168 registers, 1-2 KB of
-// spills; the 1280x720 32-spp volumetric frame 925 -> 892 ms against two at
-// 255, four 903 ms); forward media with the texture nodes two (255
-// registers; three spill more and were slower, 892 -> 915 ms on the
-// textured frame, and again with Perlin noise out of line, 745 -> 783 ms);
-// the surface adjoint three (backward pass of 16 views
-// 512² 16 spp 505 -> 487 ms); the media adjoint two.
+// The block works stage by stage: fetch the vertex, build its BSDF, and for
+// each of the (up to four) shadow rays set it up, then trace it, then the
+// continuation, with a barrier between the stages. The kernel is 150-470 KB of
+// code, more than an SM's instruction caches hold, and warps left to run on
+// their own spread over all of it: they waited for instructions 21-32 of 28-40
+// cycles per issue. Behind barriers the warps of an SM run the same few KB at
+// a time, and the wait falls to 1-4 cycles. So the block is as wide as an SM
+// has registers for (512 threads of 128) where the code is widest: media and
+// textures (one B200, without barriers at 128 threads -> 512: volumetric
+// 1280x720 16 spp 528 -> 299 ms, solid textures 8 spp 197 -> 72 ms, image
+// textures 640x480 16 spp 37.2 -> 20.3 ms; 256 threads 334, 96 and 23.4 ms).
+// Surfaces without textures need less of the code at a time and lose more to
+// the barriers: 128 threads, four blocks per SM (instanced 1080p 64 spp
+// shading 48.4 ms without barriers, 41.3 at 128, 40.5 at 256, 42.6 at 512;
+// Cornell 256x256 16 spp 1.28, 1.31, 1.37, 1.45 ms). Surface adjoint 256
+// threads (41.1 ms for 4 views 512x512 16 spp; 61.7 without barriers, 46.9 at
+// 128, 43.5 at 512).
 template <bool kVol, bool kDefer, bool kAdj, uint32_t kF>
-constexpr int shade_blocks_per_sm() {
-  if (kAdj) return kVol ? 1 : 3;
-  if (kVol) return (kF & kFeatTextures) ? 1 : 3;
-  return 4;
+constexpr uint32_t shade_threads() {
+  if (kVol || (kF & kFeatTextures)) return 512;
+  return kAdj ? 256 : 128;
+}
+template <bool kVol, bool kDefer, bool kAdj, uint32_t kF>
+constexpr uint32_t shade_blocks_per_sm() {  // 128 registers a thread
+  return 512 / shade_threads<kVol, kDefer, kAdj, kF>();
 }
 
 template <bool kVol, bool kDefer, bool kAdj, uint32_t kF>
-__global__ void __launch_bounds__(kTraceBlock, shade_blocks_per_sm<kVol, kDefer, kAdj, kF>()) k_shade(PathPool P, const WaveControl* __restrict__ ctl, HitPool H,
-                                                       PathPool Q, const JobDesc* __restrict__ jobs,
-                                                       WaveCounters* counters, ShadowQueue shadow_q,
-                                                       float* grads = nullptr, uint32_t grad_materials = 0,
-                                                       float* grid_grads = nullptr, uint32_t grid_tex = kEmpty) {
+__global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade_blocks_per_sm<kVol, kDefer, kAdj, kF>()) k_shade(
+    PathPool P, const WaveControl* __restrict__ ctl, HitPool H, PathPool Q, const JobDesc* __restrict__ jobs,
+    WaveCounters* counters, ShadowQueue shadow_q, float* grads = nullptr, uint32_t grad_materials = 0,
+    float* grid_grads = nullptr, uint32_t grid_tex = kEmpty) {
   static_assert(!(kVol && kDefer), "volume transmittance needs the path's sampler: shadow rays are traced inline");
   static_assert(!(kAdj && kDefer), "the adjoint pass traces its shadow rays inline");
+  constexpr bool kSpheres = (kF & kFeatSpheres) != 0;
   float* s_grad = nullptr;
   const uint32_t n_slots = min(grad_materials, (uint32_t)kMaxGradMaterials) * kGradParams;
   if constexpr (kAdj) {
@@ -899,100 +639,316 @@ __global__ void __launch_bounds__(kTraceBlock, shade_blocks_per_sm<kVol, kDefer,
     for (uint32_t k = threadIdx.x; k < n_slots; k += blockDim.x) s_grad[k] = 0.0f;
     __syncthreads();
   }
+  TraversalStack st;
+  if constexpr (!kDefer) {
+    YM_TRAVERSAL_SHARED_DYNAMIC(s_stack);
+    st.bind(s_stack_entries, s_stack_t);
+  } else {
+    st.sp = 0;
+    st.overflow = false;
+  }
   const bool listed = H.order != nullptr;
   const uint32_t count = listed ? min(ctl->count, counters->hit_count) : ctl->count;
   uint32_t shadow_rays = 0, tests = 0, nodes = 0;
-  bool overflow = false;
-  for (uint32_t warp_base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); warp_base < count;
-       warp_base += gridDim.x * blockDim.x) {
-  // The path slot this lane shades: the t-th listed hit, or (hits not listed
-  // by bucket) slot t itself when it holds a live path.
-  const uint32_t t_idx = warp_base + (threadIdx.x & 31u);
-  bool active = t_idx < count;
-  const uint32_t i = active ? (listed ? H.order[t_idx] : t_idx) : 0u;
-  bool alive = false;  // continues into Q
-  const uint2 pf = active ? P.pixel_flags[i] : make_uint2(kEmpty, kFlagDead);
-  if (pf.y & kFlagDead) active = false;  // a miss (already accumulated) or an empty slot
+  uint32_t* errors = &counters->errors;
+#pragma unroll 1
+  for (uint32_t block_base = blockIdx.x * blockDim.x; block_base < count; block_base += gridDim.x * blockDim.x) {
+    // The path slot this lane shades: the t-th listed hit, or (hits not listed
+    // by bucket) slot t itself when it holds a live path.
+    const uint32_t t_idx = block_base + threadIdx.x;
+    bool active = t_idx < count;
+    const uint32_t i = active ? (listed ? H.order[t_idx] : t_idx) : 0u;
+    const uint2 pf = active ? P.pixel_flags[i] : make_uint2(kEmpty, kFlagDead);
+    if (pf.y & kFlagDead) active = false;  // a miss (already accumulated) or an empty slot
+    bool alive = false;      // continues into Q
+    bool ended = false;      // a path whose radiance is complete
+    bool surface = false;    // a material vertex: next-event estimation and a BSDF continuation
+    bool volume = false;     // a volume vertex: the same with the media's phase functions
 
-  vec3 new_o, new_d, tp, rad;
-  uint32_t new_flags = 0, new_last_inst = kEmpty, new_last_tri = kEmpty;
-  PathSampler hs{0, 0u, 0u};
-  RayTransfer rt;
-  rt.record_count = 0;
-  rt.max_priority_record_index = -1;
-
-  if (active) {
-    const uint32_t job = pf.y >> kFlagJobShift;
+    vec3 new_o, new_d, tp, rad, rd;
+    uint32_t new_flags = 0, new_last_inst = kEmpty, new_last_tri = kEmpty;
+    PathSampler hs{0, 0u, 0u};
+    RayTransfer rt;
+    rt.record_count = 0;
+    rt.max_priority_record_index = -1;
+    const uint32_t job = active ? pf.y >> kFlagJobShift : 0u;
     const JobDesc& J = jobs[job];
     const uint32_t slot = J.scene_slot;
     const DeviceScene& S = c_scenes[slot];
     const RenderSetting& rs = J.setting;
-    uint32_t* errors = &counters->errors;
-    const float4 o4 = P.ray_o[i], d4 = P.ray_d[i], t4 = P.throughput[i], r4 = P.radiance[i];
-    const vec3 rd(d4.x, d4.y, d4.z);
-    (void)o4;
-    tp = vec3(t4.x, t4.y, t4.z);
-    rad = vec3(r4.x, r4.y, r4.z);
-    const uint4 s4 = P.sampler[i];
-    hs.index = (uint64_t)s4.x | ((uint64_t)s4.y << 32);
-    hs.dim = s4.z;
-    hs.aux = s4.w;
-    int depth = (int)(pf.y & kFlagDepthMask);
-    bool never_scatter = (pf.y & kFlagNeverScatter) != 0;
-    const uint32_t sample_bits = pf.y & ~(kFlagDepthMask | kFlagNeverScatter | kFlagCameraRay | kFlagDead);  // job
-    const int n_rec = P.transfer_count[i];
-    if (n_rec > 0) rt = P.transfer[i];
-    const float4 bt = H.bary_t[i];
-    const uint4 ids = H.ids[i];
-    const vec3 bary(bt.x, bt.y, bt.z);
-    const uint32_t inst_idx = ids.x, tri = ids.y;
-    const int hit_back = (int)(ids.z & 1u);
-    const bool volume_hit = kVol && (ids.z & 2u);
     const float inv_spp = 1.0f / gmax(rs.ssp, 1);
-    TraversalStack st;
-    if constexpr (!kDefer) {
-      YM_TRAVERSAL_SHARED(s_stack);
-      st.bind(s_stack_entries, s_stack_t);
-    } else {
-      st.sp = 0;
-      st.overflow = false;
+    int depth = (int)(pf.y & kFlagDepthMask);
+    const uint32_t sample_bits = pf.y & ~(kFlagDepthMask | kFlagNeverScatter | kFlagCameraRay | kFlagDead);  // job
+    uint32_t inst_idx = kEmpty, tri = kEmpty, material = 0;
+    int hit_back = 0, n_nb = 0;
+    NearbyHit nb[kMaxNearby];
+    SurfacePoint sp;           // (a volume vertex: its position in sp.p)
+    LayeredBsdf B;
+    AdjCtx adj_ctx;
+    vec3 delta(0.0f), l_total(0.0f);
+    // media of a volume vertex
+    float vw[kMaxBoundaryRecord], gs[kMaxBoundaryRecord];
+    int n_media = 0;
+    MediumAdj av{vec3(0.0f), grid_tex, grid_grads};
+
+    if (active) {
+      const float4 d4 = P.ray_d[i], t4 = P.throughput[i], r4 = P.radiance[i];
+      rd = vec3(d4.x, d4.y, d4.z);
+      tp = vec3(t4.x, t4.y, t4.z);
+      rad = vec3(r4.x, r4.y, r4.z);
+      const uint4 s4 = P.sampler[i];
+      hs.index = (uint64_t)s4.x | ((uint64_t)s4.y << 32);
+      hs.dim = s4.z;
+      hs.aux = s4.w;
+      const bool never_scatter = (pf.y & kFlagNeverScatter) != 0;
+      if (P.transfer_count[i] > 0) rt = P.transfer[i];
+      const float4 bt = H.bary_t[i];
+      const uint4 ids = H.ids[i];
+      const vec3 bary(bt.x, bt.y, bt.z);
+      inst_idx = ids.x;
+      tri = ids.y;
+      hit_back = (int)(ids.z & 1u);
+      volume = kVol && (ids.z & 2u);
+      if (kAdj) {
+        const float4 dl = J.dloss[pf.x];
+        delta = vec3(dl.x, dl.y, dl.z) * inv_spp;  // dLoss/d(this path's radiance)
+      }
+      if (volume) {
+        // Ray_shading_path_tracing volume branch (src/Shading.cu:2066-2126).
+        int vidx[kMaxBoundaryRecord];
+        n_media = current_volumes(rt, S.volume_count, vidx);
+#pragma unroll 1
+        for (int k = 0; k < n_media; ++k) {
+          gs[k] = S.volumes[vidx[k]].g;
+          vw[k] = H.vol_w[(size_t)i * kMaxBoundaryRecord + k];
+        }
+        sp.p = bary;
+        inst_idx = tri = kEmpty;
+        if (kAdj) av.scale = delta * tp;  // dLoss/d(this vertex's light), before 1/select_pdf
+      } else if (inst_idx == kEmpty) {
+        // a miss (Ray_trace_path_tracing, src/Shading.cu:1855-1864): the
+        // background when the environment light is on, then the path ends
+        if (rs.enable_env_light) rad += indirect_clamp(rs, tp * background(rd), depth);
+        ended = true;
+      } else {
+        n_nb = (int)(ids.w & 0xFFu);
+        if (ids.w & kNearbyExplicit) {
+#pragma unroll 1
+          for (int k = 0; k < n_nb; ++k) {
+            const uint4 e = H.nearby[(size_t)i * kMaxNearby + k];
+            nb[k] = NearbyHit{e.x, __uint_as_float(e.y), (int)e.z};
+          }
+        } else {
+          nb[0] = NearbyHit{inst_idx, bt.w, hit_back};
+        }
+        sp = fetch_surface<kF>(S, inst_idx, tri, bary);
+        const Instance inst = S.instances[inst_idx];
+        material = inst.material_idx;
+        if (!(material < S.material_count)) {
+          ended = true;
+        } else {
+          const Material& mat = S.materials[material];
+          uint32_t prio = 0;
+          fetch_ior(mat, &prio);
+          if (inst.treat_as_boundary ||
+              (rt.record_count != 0 && prio < rt.records[rt.max_priority_record_index].ior_priority)) {
+            // a boundary, or a lower-priority one: pass straight through, no depth consumed
+            boundary_transition(S, rt, nb, n_nb, errors);
+            new_o = offset_ray_origin(sp.p, sp.p_err, rd, sp.ng);
+            new_d = normalize(rd);
+            new_flags = flags_pack(depth, never_scatter, false, 0) | sample_bits;
+            new_last_inst = inst_idx;
+            new_last_tri = tri;
+            alive = true;
+          } else if (mat.material_type == kLightMtl) {
+            if (never_scatter) rad += indirect_clamp(rs, tp * mat.light_mtl.light_color * mat.light_mtl.intensity, depth);
+            ended = true;
+          } else {
+            surface = true;
+          }
+        }
+      }
     }
 
-    if (inst_idx == kEmpty && !volume_hit) {
-      // a miss (Ray_trace_path_tracing, src/Shading.cu:1855-1864): the
-      // background when the environment light is on, then the path ends
-      if (rs.enable_env_light) rad += indirect_clamp(rs, tp * background(rd), depth);
-      end_path<kAdj>(J, pf.x, P.path_id[i], rad, inv_spp);
-    } else if (volume_hit) {
-      // Ray_shading_path_tracing volume branch (src/Shading.cu:2066-2126).
-      float vw[kMaxBoundaryRecord], gs[kMaxBoundaryRecord];
-      int vidx[kMaxBoundaryRecord];
-      const int n = current_volumes(rt, S.volume_count, vidx);
-      for (int k = 0; k < n; ++k) {
-        gs[k] = S.volumes[vidx[k]].g;
-        vw[k] = H.vol_w[(size_t)i * kMaxBoundaryRecord + k];
+    // The layered BSDF of a material vertex.
+    __syncthreads();
+    if (surface) {
+      const DefaultMtl& md = S.materials[material].default_mtl;
+      const DefaultMtl* mp = &md;
+      DefaultMtl mt;
+      bool plain = true;
+      if constexpr ((kF & kFeatTextures) != 0) {
+        if (material_textured(md)) {
+          // textured parameters, normal or bump mapping: read at the hit
+          mt = md;
+          const TexCoord tc{sp.u, sp.v, sp.p_obj};
+          init_shading_frame_mapped(B, mt, hit_back, rd, sp, S.i_transforms[S.instances[inst_idx].transform_idx], S, tc,
+                                    errors);
+          resolve_material_textures(mt, S.textures, tc, errors);
+          mp = &mt;
+          plain = false;
+        }
       }
-      const vec3 pos = bary;
-      MediumAdj av{vec3(0.0f), grid_tex, grid_grads};
+      if (plain) init_shading_frame(B, hit_back, rd, sp.ng, sp.ns, sp.dpdu, sp.dpdv);
+      init_layered_lobes(B, *mp, rd, hit_back, ray_ior(rt), ex_ior(rt, inst_idx));
       if constexpr (kAdj) {
-        const float4 dl = J.dloss[pf.x];
-        av.scale = vec3(dl.x, dl.y, dl.z) * inv_spp * tp;  // dLoss/d(this vertex's light), before 1/select_pdf
+        const float4 lt = J.path_radiance[P.path_id[i]];
+        l_total = vec3(lt.x, lt.y, lt.z);
+        init_adjoint(adj_ctx, B, *mp);
+        adj_ctx.weight = delta * tp;
       }
-      if (rs.enable_distant_light)
-        rad += indirect_clamp(rs, tp * eval_volume_lights<kF, kAdj>(slot, st, true, n, gs, vw, rd, rt, pos, hs,
-                                                                    &shadow_rays, &tests, &nodes, errors,
-                                                                    kAdj ? &av : nullptr), depth);
-      if (rs.enable_shape_light)
-        rad += indirect_clamp(rs, tp * eval_volume_lights<kF, kAdj>(slot, st, false, n, gs, vw, rd, rt, pos, hs,
-                                                                    &shadow_rays, &tests, &nodes, errors,
-                                                                    kAdj ? &av : nullptr), depth);
-      vec3 wi;
-      float pdf = 0.0f, pw = 0.0f;
-      float u0, u1;
+    }
+    const vec3 wo = surface ? B.to_local(-rd) : vec3(0.0f);
+
+    // Next-event estimation: EvalDistantLight / EvalShapeLight (src/Shading.cu:83-198,
+    // 294-417) at material vertices, EvalVolumeDistantLight / EvalVolumeShapeLight
+    // (:202-291, 419-513) at volume vertices. Two kinds of light, and for each
+    // a direction sampled from the light (pass 0) and one from the BSDF or the
+    // phase functions (pass 1).
+#pragma unroll 1
+    for (int kind = 0; kind < 2; ++kind) {
+      const bool distant = kind == 0;
+      const bool on = (surface || (volume && n_media > 0)) &&
+                      (distant ? rs.enable_distant_light && S.distant_light_count > 0
+                               : rs.enable_shape_light != 0 && S.shape_light_count > 0);
+      if (!__syncthreads_or(on)) continue;
+      ChosenLight L;
+      vec3 direct(0.0f);
+      if (on) choose_light<kF>(S, distant, hs, L);
+#pragma unroll 1
+      for (int pass = 0; pass < 2; ++pass) {
+        LightSample q{vec3(0.0f), vec3(0.0f), vec3(0.0f), vec3(0.0f), vec3(0.0f), 0.0f};
+        vec3 f(0.0f), lwi(0.0f), so(0.0f);
+        float spdf = 0.0f, maxd = kTMax;  // spdf: of the BSDF or the phase functions
+        bool ok = on, tb = false;
+        if (on) {
+          float u0, u1, u2 = 0.0f;
+          sample2d(hs, S, &u0, &u1);
+          if (surface && pass == 1) u2 = sample1d(hs, S);
+          if (pass == 0) {
+            ok = sample_chosen_light<kF>(S, L, sp.p, u0, u1, q);
+            if (ok) {
+              if (!kVol || surface) {
+                lwi = B.to_local(q.dir);
+                f = bsdf_eval(B, wo, lwi, &spdf);
+              } else {
+                f = vec3(eval_mixed_phases(vw, gs, n_media, -rd, q.dir, &spdf));
+              }
+              ok = max_component(f) > kMinColorEps;
+            }
+          } else {
+            if (!kVol || surface) {
+              ok = bsdf_sample(B, wo, &f, &lwi, &spdf, u0, u1, u2);
+              if (ok) q.dir = B.to_world(lwi);
+            } else {
+              float pw = 0.0f;
+              ok = sample_mixed_phases(vw, gs, n_media, u0, u1, -rd, &pw, &q.dir, &spdf);
+              f = vec3(pw);
+            }
+            if (ok) {
+              eval_chosen_light<kF>(S, L, sp.p, q);
+              ok = max_component(q.Li) > kMinColorEps;
+            }
+          }
+          so = sp.p;
+          if (ok && surface) {
+            tb = dot(-rd, sp.ng) * dot(q.dir, sp.ng) < 0.0f;
+            if (same_hemisphere(wo, lwi) ? tb : !tb) ok = false;
+            else so = offset_ray_origin(sp.p, sp.p_err, q.dir, sp.ng);
+          }
+          if (ok && !distant) maxd = length(offset_ray_origin(q.pos, q.err, -q.dir, q.ng) - sp.p) * kShadowRayClamp;
+        }
+        float mis = 0.0f;
+        vec3 fc(0.0f), Lc(0.0f);
+        if (ok) {
+          ++shadow_rays;
+          mis = power_heuristic(pass == 0 ? q.pdf : spdf, pass == 0 ? spdf : q.pdf);
+          fc = vmin(f, vec3(kMaxColorClamp));
+          Lc = vmin(q.Li, vec3(kMaxColorClamp));
+        }
+        if constexpr (kDefer) {
+          // the light-selection pdf enters as a factor here and as a quotient for distant lights
+          if (ok) {
+            const ShadowEmit em{shadow_q, &counters->shadow_count, errors, pf.x, job, P.path_id[i], tp * inv_spp};
+            const float mul = distant ? 1.0f : safe_rcp(L.select_pdf), div = distant ? L.select_pdf : 1.0f;
+            emit_shadow_ray(em, so, normalize(q.dir), maxd, ((mis * vec3(1.0f) * fc * Lc) * mul) / div);
+          }
+          __syncthreads();
+        } else {
+          __syncthreads();
+          if (ok) {
+            const vec3 dir = normalize(q.dir);
+            if (!trace_occluded_impl<kSpheres>(slot, st, so, dir, maxd, &tests, &nodes)) {
+              vec3 tr(1.0f);
+              const PathSampler hs0 = hs;
+              const bool media = kVol && (volume || rs.enable_volume_scattering);
+              if (media) {
+                RayTransfer srt = rt;
+                if (tb) boundary_transition(S, srt, nb, n_nb, errors);
+                tr = trace_tr<kF>(slot, st, so, dir, maxd, inst_idx, tri, srt, hs, errors, &tests, &nodes);
+              }
+              const vec3 contrib = mis * tr * fc * Lc;
+              direct += contrib;
+              if constexpr (kAdj) {
+                const float mul = distant || volume ? 1.0f : safe_rcp(L.select_pdf);
+                const float div = distant || volume ? L.select_pdf : 1.0f;
+                if (kVol && grid_grads && media && (!volume || L.select_pdf > 0.0f)) {
+                  // the transmittance's density-grid terms: replay its tracking with the
+                  // same samples, weighted by this ray's share of dLoss
+                  const MediumAdj am{volume ? av.scale * contrib / L.select_pdf : adj_ctx.weight * (mul / div) * contrib,
+                                     grid_tex, grid_grads};
+                  if (max_component(vabs(am.scale)) > 0.0f) {
+                    RayTransfer srt = rt;
+                    if (tb) boundary_transition(S, srt, nb, n_nb, errors);
+                    PathSampler h2 = hs0;
+                    trace_tr<kF, true>(slot, st, so, dir, maxd, inst_idx, tri, srt, h2, errors, &tests, &nodes, &am);
+                  }
+                }
+                // d(direct)/dp = mis * tr * fc * (df/dp)/f * Lc, scaled like the estimator
+                if (surface)
+                  add_relative_grads(&adj_ctx, B, wo, B.to_local(q.dir), adj_ctx.weight * (mul / div), contrib);
+              }
+            }
+          }
+          __syncthreads();
+        }
+      }
+      if (on) {
+        const vec3 e = distant || (kVol && volume) ? (L.select_pdf > 0.0f ? direct / L.select_pdf : vec3(0.0f))
+                                                   : direct * safe_rcp(L.select_pdf);
+        rad += indirect_clamp(rs, tp * e, depth);
+      }
+    }
+
+    // The continuation: a direction from the BSDF or the phase functions.
+    if (surface || (kVol && volume)) {
+      float u0, u1, u2 = 0.0f;
       sample2d(hs, S, &u0, &u1);
-      bool terminate = !sample_mixed_phases(vw, gs, n, u0, u1, -rd, &pw, &wi, &pdf);
-      if (!terminate) {
-        tp *= pw;
+      vec3 w(0.0f), wi(0.0f);
+      float pdf = 0.0f;
+      bool valid;
+      if (!kVol || surface) {
+        u2 = sample1d(hs, S);
+        valid = bsdf_sample(B, wo, &w, &wi, &pdf, u0, u1, u2);
+      } else {
+        float pw = 0.0f;
+        valid = sample_mixed_phases(vw, gs, n_media, u0, u1, -rd, &pw, &wi, &pdf);
+        w = vec3(pw);
+      }
+      if constexpr (kAdj) {
+        if (surface) {
+          // the radiance gathered after this vertex, through the sampled BSDF value
+          if (valid) add_relative_grads(&adj_ctx, B, wo, wi, delta, l_total - rad);
+          for (int k = 0; k < kGradParams; ++k) {
+            if (adj_ctx.g[k] == 0.0f) continue;
+            if (material * kGradParams + k < n_slots) atomicAdd(&s_grad[material * kGradParams + k], adj_ctx.g[k]);
+            else if (material < grad_materials) atomicAdd(&grads[material * kGradParams + k], adj_ctx.g[k]);
+          }
+        }
+      }
+      bool terminate = !valid;
+      if (valid) {
+        tp *= w;
         float rr = gmax(tp.x, gmax(tp.y, tp.z));
         rr = gmin(rr, 1.0f);
         if (depth + 1 > rs.ray_depth) {
@@ -1001,177 +957,42 @@ __global__ void __launch_bounds__(kTraceBlock, shade_blocks_per_sm<kVol, kDefer,
         }
       }
       if (!terminate) {
-        new_o = pos;
-        new_d = normalize(wi);
-        depth += 1;
-        if (depth > kMaxRayDepth) {
-          terminate = true;
-        } else {
-          new_flags = flags_pack(depth, false, false, 0) | sample_bits;
-          new_last_inst = kEmpty;
-          new_last_tri = kEmpty;
-          alive = true;
-        }
-      }
-      if (terminate) end_path<kAdj>(J, pf.x, P.path_id[i], rad, inv_spp);
-    } else {
-      NearbyHit nb[kMaxNearby];
-      const int n_nb = (int)(ids.w & 0xFFu);
-      if (ids.w & kNearbyExplicit) {
-        for (int k = 0; k < n_nb; ++k) {
-          const uint4 e = H.nearby[(size_t)i * kMaxNearby + k];
-          nb[k] = NearbyHit{e.x, __uint_as_float(e.y), (int)e.z};
-        }
-      } else {
-        nb[0] = NearbyHit{inst_idx, bt.w, hit_back};
-      }
-      const SurfacePoint sp = fetch_surface<kF>(S, inst_idx, tri, bary);
-      const Instance inst = S.instances[inst_idx];
-      bool done = false;
-      if (!(inst.material_idx < S.material_count)) {
-        end_path<kAdj>(J, pf.x, P.path_id[i], rad, inv_spp);
-        done = true;
-      }
-      const Material& mat = S.materials[done ? 0 : inst.material_idx];
-      uint32_t prio = 0;
-      if (!done) fetch_ior(mat, &prio);
-      if (!done && rt.record_count != 0 && prio < rt.records[rt.max_priority_record_index].ior_priority) {
-        // lower-priority boundary: pass straight through, no depth consumed
-        boundary_transition(S, rt, nb, n_nb, errors);
-        new_o = offset_ray_origin(sp.p, sp.p_err, rd, sp.ng);
-        new_d = normalize(rd);
-        new_flags = flags_pack(depth, never_scatter, false, 0) | sample_bits;
-        new_last_inst = inst_idx;
-        new_last_tri = tri;
-        alive = true;
-        done = true;
-      }
-      if (!done && inst.treat_as_boundary) {
-        boundary_transition(S, rt, nb, n_nb, errors);
-        new_o = offset_ray_origin(sp.p, sp.p_err, rd, sp.ng);
-        new_d = normalize(rd);
-        new_flags = flags_pack(depth, never_scatter, false, 0) | sample_bits;
-        new_last_inst = inst_idx;
-        new_last_tri = tri;
-        alive = true;
-        done = true;
-      }
-      if (!done && mat.material_type == kLightMtl) {
-        if (never_scatter) rad += indirect_clamp(rs, tp * mat.light_mtl.light_color * mat.light_mtl.intensity, depth);
-        end_path<kAdj>(J, pf.x, P.path_id[i], rad, inv_spp);
-        done = true;
-      }
-      if (!done) {
-        LayeredBsdf B;
-        const DefaultMtl* mp = &mat.default_mtl;
-        DefaultMtl mt;
-        if constexpr ((kF & kFeatTextures) != 0) {
-          if (material_textured(mat.default_mtl)) {
-            // textured parameters, normal or bump mapping: read at the hit
-            mt = mat.default_mtl;
-            const TexCoord tc{sp.u, sp.v, sp.p_obj};
-            init_shading_frame_mapped(B, mt, hit_back, rd, sp, S.i_transforms[inst.transform_idx], S, tc, errors);
-            resolve_material_textures(mt, S.textures, tc, errors);
-            mp = &mt;
+        new_o = sp.p;
+        vec3 nd = wi;
+        if (!kVol || surface) {
+          nd = B.to_world(wi);
+          const bool tb = dot(-rd, sp.ng) * dot(nd, sp.ng) < 0.0f;
+          if (same_hemisphere(wo, wi) ? tb : !tb) {
+            terminate = true;
           } else {
-            init_shading_frame(B, hit_back, rd, sp.ng, sp.ns, sp.dpdu, sp.dpdv);
-          }
-        } else {
-          init_shading_frame(B, hit_back, rd, sp.ng, sp.ns, sp.dpdu, sp.dpdv);
-        }
-        init_layered_lobes(B, *mp, rd, hit_back, ray_ior(rt), ex_ior(rt, inst_idx));
-        const SurfaceNee nc{rd, sp.p, sp.p_err, sp.ng, inst_idx, tri, &rt, nb, n_nb, rs.enable_volume_scattering != 0,
-                            slot};
-        const ShadowEmit em{shadow_q, &counters->shadow_count, errors, pf.x, job, P.path_id[i], tp * inv_spp};
-        AdjCtx adj_ctx;
-        AdjCtx* adj = nullptr;
-        vec3 delta(0.0f), l_total(0.0f);
-        if constexpr (kAdj) {
-          const float4 dl = J.dloss[pf.x];
-          const float4 lt = J.path_radiance[P.path_id[i]];
-          delta = vec3(dl.x, dl.y, dl.z) * inv_spp;  // dLoss/d(this path's radiance)
-          l_total = vec3(lt.x, lt.y, lt.z);
-          init_adjoint(adj_ctx, B, *mp);
-          adj_ctx.weight = delta * tp;
-          adj_ctx.grid_grads = grid_grads;
-          adj_ctx.grid_tex = grid_tex;
-          adj = &adj_ctx;
-        }
-        if (rs.enable_distant_light)
-          rad += indirect_clamp(
-              rs, tp * eval_distant_light<kVol, kDefer, kF>(S, st, B, nc, em, hs, &shadow_rays, &tests, &nodes, errors, adj),
-              depth);
-        if (rs.enable_shape_light)
-          rad += indirect_clamp(
-              rs, tp * eval_shape_light<kVol, kDefer, kF>(S, st, B, nc, em, hs, &shadow_rays, &tests, &nodes, errors, adj),
-              depth);
-        const vec3 wo = B.to_local(-rd);
-        vec3 w, wi;
-        float pdf = 0.0f;
-        float u0, u1, u2;
-        sample3d(hs, S, &u0, &u1, &u2);
-        const bool valid = bsdf_sample(B, wo, &w, &wi, &pdf, u0, u1, u2);
-        if constexpr (kAdj) {
-          // the radiance gathered after this vertex, through the sampled BSDF value
-          if (valid) add_relative_grads(&adj_ctx, B, wo, wi, delta, l_total - rad);
-          const uint32_t m = inst.material_idx;
-          for (int k = 0; k < kGradParams; ++k) {
-            if (adj_ctx.g[k] == 0.0f) continue;
-            if (m * kGradParams + k < n_slots) atomicAdd(&s_grad[m * kGradParams + k], adj_ctx.g[k]);
-            else if (m < grad_materials) atomicAdd(&grads[m * kGradParams + k], adj_ctx.g[k]);
+            if (tb) boundary_transition(S, rt, nb, n_nb, errors);
+            new_o = offset_ray_origin(sp.p, sp.p_err, nd, sp.ng);
           }
         }
-        if (!valid) {
-          end_path<kAdj>(J, pf.x, P.path_id[i], rad, inv_spp);
-        } else {
-          tp *= w;
-          float rr = gmax(tp.x, gmax(tp.y, tp.z));
-          rr = gmin(rr, 1.0f);
-          bool terminate = false;
-          if (depth + 1 > rs.ray_depth) {
-            if (rs.enable_russian_roulette && sample1d(hs, S) < rr) tp /= gmax(rr, kMinColorEps);
-            else terminate = true;
-          }
-          if (!terminate) {
-            const vec3 nd = B.to_world(wi);
-            const bool tb = dot(-rd, sp.ng) * dot(nd, sp.ng) < 0.0f;
-            const bool invalid = (!same_hemisphere(wo, wi) && !tb) || (same_hemisphere(wo, wi) && tb);
-            if (invalid) {
-              terminate = true;
-            } else {
-              if (tb) boundary_transition(S, rt, nb, n_nb, errors);
-              new_o = offset_ray_origin(sp.p, sp.p_err, nd, sp.ng);
-              new_d = normalize(nd);
-              never_scatter = false;
-              depth += 1;
-              if (depth > kMaxRayDepth) {
-                terminate = true;
-              } else {
-                new_flags = flags_pack(depth, false, false, 0) | sample_bits;
-                new_last_inst = inst_idx;
-                new_last_tri = tri;
-                alive = true;
-              }
-            }
-          }
-          if (terminate) end_path<kAdj>(J, pf.x, P.path_id[i], rad, inv_spp);
-        }
+        new_d = normalize(nd);
+        depth += 1;
+        if (depth > kMaxRayDepth) terminate = true;
+        new_flags = flags_pack(depth, false, false, 0) | sample_bits;
+        new_last_inst = inst_idx;
+        new_last_tri = tri;
+        alive = !terminate;
+      }
+      ended = terminate;
+    }
+    if (ended) end_path<kAdj>(J, pf.x, P.path_id[i], rad, inv_spp);
+
+    const uint32_t q_slot = warp_append(&counters->next_count, alive);
+    if (alive) {
+      if (q_slot < Q.capacity) {
+        store_path(Q, q_slot, new_o, new_d, tp, rad, pf.x, new_flags, new_last_inst, new_last_tri, hs, P.path_id[i]);
+        Q.transfer_count[q_slot] = (uint8_t)rt.record_count;
+        if (rt.record_count > 0) Q.transfer[q_slot] = rt;
+      } else {
+        atomicOr(&counters->errors, (uint32_t)kDevErrQueue);
       }
     }
-    overflow = overflow || st.overflow;
   }
-  const uint32_t slot = warp_append(&counters->next_count, alive);
-  if (alive) {
-    if (slot < Q.capacity) {
-      store_path(Q, slot, new_o, new_d, tp, rad, pf.x, new_flags, new_last_inst, new_last_tri, hs, P.path_id[i]);
-      Q.transfer_count[slot] = (uint8_t)rt.record_count;
-      if (rt.record_count > 0) Q.transfer[slot] = rt;
-    } else {
-      atomicOr(&counters->errors, (uint32_t)kDevErrQueue);
-    }
-  }
-  }
-  if (overflow) atomicOr(&counters->errors, (uint32_t)kDevErrStack);
+  if (st.overflow) atomicOr(&counters->errors, (uint32_t)kDevErrStack);
   uint32_t s_sum = shadow_rays, t_sum = tests, n_sum = nodes;
   for (int off = 16; off > 0; off >>= 1) {
     s_sum += __shfl_down_sync(0xFFFFFFFFu, s_sum, off);
@@ -1188,6 +1009,25 @@ __global__ void __launch_bounds__(kTraceBlock, shade_blocks_per_sm<kVol, kDefer,
     for (uint32_t k = threadIdx.x; k < n_slots; k += blockDim.x)
       if (s_grad[k] != 0.0f) atomicAdd(&grads[k], s_grad[k]);
   }
+}
+
+// Lets a k_shade instantiation that traces its shadow rays inline take its
+// block's traversal stacks in dynamic shared memory (more than the default 48 KB).
+template <bool kVol, bool kAdj, uint32_t kF>
+static void allow_shade_shared() {
+  cudaFuncSetAttribute(k_shade<kVol, false, kAdj, kF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)traversal_shared_bytes(shade_threads<kVol, false, kAdj, kF>()));
+}
+
+// Launches k_shade over the wave (one thread per pool slot).
+template <bool kVol, bool kDefer, bool kAdj, uint32_t kF>
+void launch_shade(const WaveArgs& w, const ShadowQueue& q, float* grads = nullptr, uint32_t grad_materials = 0,
+                  float* grid_grads = nullptr, uint32_t grid_tex = kEmpty) {
+  constexpr uint32_t threads = shade_threads<kVol, kDefer, kAdj, kF>();
+  const uint32_t blocks = (w.blocks * kTraceBlock + threads - 1) / threads;
+  const size_t shared = kDefer ? 0 : traversal_shared_bytes(threads);
+  k_shade<kVol, kDefer, kAdj, kF><<<blocks, threads, shared, w.stream>>>(w.A, w.ctl, w.H, w.B, w.jobs, w.counters, q,
+                                                                         grads, grad_materials, grid_grads, grid_tex);
 }
 
 // ------------------------------------------------------------- connect ---
