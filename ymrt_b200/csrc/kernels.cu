@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_debug_trace(uint32_t slot, int 
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   TraversalStack st;
-  st.bind(s_stack_entries, s_stack_t);
+  st.bind(s_stack);
   const vec3 o(origin[3 * i], origin[3 * i + 1], origin[3 * i + 2]);
   const vec3 d = normalize(vec3(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]));
   ClosestHit ch;
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_debug_occluded(uint32_t slot, i
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   TraversalStack st;
-  st.bind(s_stack_entries, s_stack_t);
+  st.bind(s_stack);
   const vec3 o(origin[3 * i], origin[3 * i + 1], origin[3 * i + 2]);
   const vec3 d = normalize(vec3(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]));
   uint32_t tests = 0, nodes = 0;
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_editor_view(int slot, int width
   RayTransfer rt = cam.transfer;
   uint32_t last_inst = kEmpty, last_tri = kEmpty;
   TraversalStack st;
-  st.bind(s_stack_entries, s_stack_t);
+  st.bind(s_stack);
   uint32_t tests = 0, nodes = 0;
   vec3 col(0.0f);
   bool done = false;

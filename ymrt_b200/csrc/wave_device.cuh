@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kMaxTraceBlock, 4 * kTraceBlock / kMaxTraceBlo
     const vec3 o(o4.x, o4.y, o4.z), d(d4.x, d4.y, d4.z);
     const uint2 lh = P.last_hit[i];
     TraversalStack st;
-    st.bind(s_stack_entries, s_stack_t);
+    st.bind(s_stack);
     ClosestHit ch;
     bool hit = trace_closest_impl<(kF & kFeatSpheres) != 0>(slot, st, o, d, kTMax, lh.x, lh.y, false, &ch, &tests, &nodes);
     overflow = overflow || st.overflow;
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
   TraversalStack st;
   if constexpr (!kDefer) {
     YM_TRAVERSAL_SHARED_DYNAMIC(s_stack);
-    st.bind(s_stack_entries, s_stack_t);
+    st.bind(s_stack);
   } else {
     st.sp = 0;
     st.overflow = false;
@@ -1042,9 +1042,9 @@ template <uint32_t kF>
 __global__ void __launch_bounds__(kMaxTraceBlock, kConnectBlocksPerSm * kTraceBlock / kMaxTraceBlock) k_connect(ShadowQueue Q,
                                                                              const JobDesc* __restrict__ jobs,
                                                                              WaveCounters* counters) {
-  extern __shared__ __align__(16) uint32_t s_stack[];  // occluded_shared_bytes(blockDim.x)
+  extern __shared__ __align__(16) uint32_t s_occ[];  // occluded_shared_bytes(blockDim.x)
   OccStack st;
-  st.bind(s_stack);
+  st.bind(s_occ);
   OccWalk w;
   const uint32_t n = min(counters->shadow_count, Q.capacity);
   const int lane = threadIdx.x & 31;
