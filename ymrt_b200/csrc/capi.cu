@@ -303,7 +303,7 @@ struct ymrt_scene {
     bool prepared = false;
     int cur = 0;                             // which of the pairs below holds the current order
     DeviceBuffer inst[2], bucket[2], file_idx[2];
-    DeviceBuffer scales, items, nodes, mid, kind, left, stack, wide, prims, offsets, inside, camera, counts;
+    DeviceBuffer scales, items, nodes, mid, kind, left, stack, wide, prims, slots, offsets, inside, camera, counts;
   } top;
 
   template <typename T>
@@ -752,6 +752,12 @@ int ymrt_scene_upload(ymrt_context* ctx, const ymrt_host_scene* hs, const uint32
   std::vector<uint8_t> buckets(s.instances.size());
   for (size_t i = 0; i < s.instances.size(); ++i) buckets[i] = (uint8_t)shading_bucket(s, s.instances[i]);
   UP(buckets, inst_bucket);
+  std::vector<InstanceSlot> slots(s.tlas_prims.size());
+  for (size_t k = 0; k < slots.size(); ++k) {
+    const Instance& inst = s.instances[s.tlas_prims[k]];
+    slots[k] = make_instance_slot(s.tlas_prims[k], inst, s.i_transforms[inst.transform_idx], s.geo_desc[inst.geometry_idx]);
+  }
+  UP(slots, inst_slots);
 #undef UP
   sc->pack(halton_perm, perm_len, &D.halton_perm);
   if (e == cudaSuccess) e = sc->pack_commit();
@@ -1411,6 +1417,7 @@ int ymrt_scene_set_transforms(ymrt_scene* sc, uint32_t first, uint32_t count, co
     if (e == cudaSuccess) e = T.stack.ensure(sizeof(uint32_t) * 2 * (7 * nb + 2));
     if (e == cudaSuccess) e = T.wide.ensure(sizeof(WideNode) * std::max<size_t>(2 * (size_t)n, 2));
     if (e == cudaSuccess) e = T.prims.ensure(sizeof(uint32_t) * n);
+    if (e == cudaSuccess) e = T.slots.ensure(sizeof(InstanceSlot) * n);
     if (e == cudaSuccess) e = T.offsets.ensure(sizeof(uint32_t) * n);
     if (e == cudaSuccess) e = T.inside.ensure(n);
     if (e == cudaSuccess) e = T.camera.ensure(sizeof(RayTransfer));
@@ -1455,6 +1462,7 @@ int ymrt_scene_set_transforms(ymrt_scene* sc, uint32_t first, uint32_t count, co
   b.stack = T.stack.as<uint32_t>();
   b.wide = T.wide.as<WideNode>();
   b.prims = T.prims.as<uint32_t>();
+  b.slots = T.slots.as<InstanceSlot>();
   b.lights = const_cast<ShapeLight*>(D.shape_lights);
   b.light_table = const_cast<float*>(D.shape_light_table);
   b.light_count = D.shape_light_count;
@@ -1478,6 +1486,7 @@ int ymrt_scene_set_transforms(ymrt_scene* sc, uint32_t first, uint32_t count, co
   D.inst_bucket = T.bucket[o].as<uint8_t>();
   D.tlas_nodes = T.wide.as<WideNode>();
   D.tlas_prims = T.prims.as<uint32_t>();
+  D.inst_slots = T.slots.as<InstanceSlot>();
   D.camera.transfer = rt;
   return YMRT_OK;
 }

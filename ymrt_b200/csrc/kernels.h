@@ -274,6 +274,7 @@ struct TlasBuild {
   // outputs
   WideNode* wide;         // top-level nodes (at most 2n)
   uint32_t* prims;        // n: instance per top-level leaf slot
+  InstanceSlot* slots;    // n: the same slots' instances for the traversal
   ShapeLight* lights;
   float* light_table;
   uint32_t light_count;   // entries the table holds (an edit keeps the count)

@@ -230,6 +230,16 @@ __global__ void __launch_bounds__(kCameraThreads) k_camera_inside(TlasBuild b, v
   if (threadIdx.x == 0) b.inside[i] = (any_fwd && any_bwd) ? 1 : 0;
 }
 
+// The traversal's record of each top-level leaf slot (after the reorder).
+__global__ void k_instance_slots(TlasBuild b) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= b.n) return;
+  const uint32_t i = b.prims[k];
+  if (i >= b.n) return;
+  const Instance inst = b.instances_out[i];
+  b.slots[k] = make_instance_slot(i, inst, b.i_transforms[inst.transform_idx], b.geometries[inst.geometry_idx]);
+}
+
 __global__ void k_camera_stack(TlasBuild b) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   RayTransfer rt{};  // records past record_count stay zero, as on the host
@@ -262,6 +272,7 @@ void launch_tlas_rebuild(const TlasBuild& b, uint32_t max_leaf, vec3 cam_pos, ve
   k_tlas_binary<<<1, kBinaryThreads, 0, stream>>>(b);
   k_tlas_wide<<<1, 32, 0, stream>>>(b, max_leaf);
   k_tlas_reorder<<<blocks, 128, 0, stream>>>(b);
+  k_instance_slots<<<blocks, 128, 0, stream>>>(b);
   k_light_count<<<blocks, 128, 0, stream>>>(b);
   k_light_offsets<<<1, 32, 0, stream>>>(b);
   k_light_fill<<<blocks, 128, 0, stream>>>(b);

@@ -240,6 +240,32 @@ struct GeometryDesc {
   float radius;             // sphere radius (Sphere::radius)
 };
 
+// What a traversal reads to enter an instance, one 64-byte record per leaf
+// slot of the top level (four 128-bit loads that need no other load first,
+// where the instance, its inverse transform and its geometry are a chain of
+// three): the rows of the world-to-object matrix, the instance, and its
+// geometry's root and triangles (a sphere: its radius).
+struct alignas(16) InstanceSlot {
+  float row[3][4];       // row r of the matrix: columns 0-3
+  uint32_t inst;
+  uint32_t node_offset;
+  uint32_t wtri_offset;  // a sphere: its radius (bits)
+  uint32_t flags;        // kSlot*
+};
+static_assert(sizeof(InstanceSlot) == 64, "InstanceSlot is four 16-byte words");
+constexpr uint32_t kSlotBoundary = 1, kSlotSphere = 2;
+YM_HD InstanceSlot make_instance_slot(uint32_t index, const Instance& inst, const mat4& world_to_object,
+                                      const GeometryDesc& g) {
+  InstanceSlot s;
+  for (int r = 0; r < 3; ++r)
+    for (int c = 0; c < 4; ++c) s.row[r][c] = world_to_object.m[c][r];
+  s.inst = index;
+  s.node_offset = g.node_offset;
+  s.wtri_offset = g.kind == kGeoSphere ? f2u(g.radius) : g.wtri_offset;
+  s.flags = (inst.treat_as_boundary ? kSlotBoundary : 0u) | (g.kind == kGeoSphere ? kSlotSphere : 0u);
+  return s;
+}
+
 // Everything the kernels read, as device pointers.
 // RenderSetting::sampler_type values (src/RandomSampler.cuh:617-620).
 constexpr uint32_t kSamplerPcg = 0, kSamplerHalton = 1, kSamplerSobol = 2;
@@ -255,6 +281,7 @@ struct DeviceScene {
   // top-level BVH over instances
   const WideNode* tlas_nodes;
   const uint32_t* tlas_prims;   // instance index per TLAS leaf slot
+  const InstanceSlot* inst_slots;  // the same slots' instances, as the traversal enters them
   // meshes
   uint32_t geometry_count;
   const GeometryDesc* geometries;
