@@ -90,6 +90,9 @@ struct ymrt_context {
     graph_key.clear();
   }
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
+  // the branch of the captured wave loop that traces deferred shadow rays
+  cudaStream_t connect_stream = nullptr;
+  cudaEvent_t ev_fork[2] = {nullptr, nullptr};
   bool profiling = false;
   cudaEvent_t ev_stage[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   WaveCounters batch_counters{};  // frame totals across the launch groups of one batch
@@ -198,7 +201,7 @@ struct ymrt_context {
     cudaError_t e = shadow_buf.ensure(n * (3 * sizeof(float4) + sizeof(uint32_t)));
     if (e != cudaSuccess) return cuda_fail(e, "allocating shadow-ray queue");
     float4* q = shadow_buf.as<float4>();
-    shadow_queue = ShadowQueue{q, q + n, q + 2 * n, reinterpret_cast<uint32_t*>(q + 3 * n), (uint32_t)n};
+    shadow_queue = ShadowQueue{q, q + n, q + 2 * n, reinterpret_cast<uint32_t*>(q + 3 * n), (uint32_t)n, 0u};
     return YMRT_OK;
   }
 };
@@ -447,6 +450,11 @@ int ymrt_create(int device_ordinal, ymrt_context** out) {
     return ctx->cuda_fail(e, "cudaEventCreate");
   for (auto& ev : ctx->ev_stage)
     if ((e = cudaEventCreate(&ev)) != cudaSuccess) return ctx->cuda_fail(e, "cudaEventCreate");
+  if ((e = cudaStreamCreateWithFlags(&ctx->connect_stream, cudaStreamNonBlocking)) != cudaSuccess)
+    return ctx->cuda_fail(e, "cudaStreamCreate");
+  for (auto& ev : ctx->ev_fork)
+    if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
+      return ctx->cuda_fail(e, "cudaEventCreate");
   if ((e = cudaMallocHost(&ctx->counters_host, sizeof(WaveCounters))) != cudaSuccess)
     return ctx->cuda_fail(e, "cudaMallocHost");
   if ((e = cudaMallocHost(&ctx->ctl_host, sizeof(WaveControl))) != cudaSuccess)
@@ -475,6 +483,9 @@ void ymrt_destroy(ymrt_context* ctx) {
   if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);
   for (auto& ev : ctx->ev_stage)
     if (ev) cudaEventDestroy(ev);
+  for (auto& ev : ctx->ev_fork)
+    if (ev) cudaEventDestroy(ev);
+  if (ctx->connect_stream) cudaStreamDestroy(ctx->connect_stream);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
@@ -986,11 +997,24 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
       cudaGraph_t body = params.conditional.phGraph_out[0];
       e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
       if (e == cudaSuccess) {
-        launch_wave(M.pool[0], M.pool[1], M.hits, M.ctl, M.jobs, (uint32_t)jobs.size(), M.counters, o, nullptr, st,
-                    (unsigned long long)cond);
-        launch_wave(M.pool[1], M.pool[0], M.hits, M.ctl, M.jobs, (uint32_t)jobs.size(), M.counters, o, nullptr, st,
-                    (unsigned long long)cond);
+        const bool forks = defers_shadows(o);
+        for (uint32_t turn = 0; turn < 2; ++turn) {
+          const WaveFork fork{ctx->connect_stream, ctx->ev_fork[0], ctx->ev_fork[1], turn};
+          launch_wave(M.pool[turn], M.pool[turn ^ 1u], M.hits, M.ctl, M.jobs, (uint32_t)jobs.size(), M.counters, o,
+                      nullptr, st, (unsigned long long)cond, forks ? &fork : nullptr);
+        }
         e = cudaStreamEndCapture(st, &body);
+        if (e == cudaSuccess && forks) {
+          // the shadow rays of the last wave, after the loop (the loop's body
+          // ends with turn 1; a frame that ends in turn 0 leaves turn 1 empty,
+          // which has traced turn 0's)
+          e = cudaStreamBeginCaptureToGraph(st, g, &node, nullptr, 1, cudaStreamCaptureModeRelaxed);
+          if (e == cudaSuccess) {
+            launch_connect(o.shadow_queue, 1u, M.jobs, M.counters, o, st);
+            cudaGraph_t captured = nullptr;
+            e = cudaStreamEndCapture(st, &captured);
+          }
+        }
       }
       cudaGraphExec_t exec = nullptr;
       if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);

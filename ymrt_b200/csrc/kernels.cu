@@ -451,13 +451,15 @@ cudaError_t upload_constants(const DeviceScene* scenes, const uint32_t* slots, u
 
 // Start of a wave: the continuing paths left by the previous wave, the new
 // paths to generate (as many as fit), and the per-wave counters cleared.
-__global__ void k_plan(WaveControl* ctl, WaveCounters* counters) {
+__global__ void k_plan(WaveControl* ctl, WaveCounters* counters, uint32_t turn) {
   __shared__ uint32_t s_live;
   if (threadIdx.x == 0) s_live = counters->next_count;
   __syncthreads();
   uint32_t* words = reinterpret_cast<uint32_t*>(counters);
   for (uint32_t k = threadIdx.x; k < (uint32_t)(kWaveClearBytes / sizeof(uint32_t)); k += blockDim.x) words[k] = 0u;
   if (threadIdx.x == 0) {
+    counters->shadow_count[turn] = 0u;
+    counters->shadow_cursor[turn] = 0u;
     const uint32_t live = ctl->more ? s_live : 0u;
     const unsigned long long left = ctl->more ? ctl->total - ctl->cursor : 0ull;
     const uint32_t room = ctl->capacity > live ? ctl->capacity - live : 0u;
@@ -637,11 +639,9 @@ struct PersistentGrids {
 };
 PersistentGrids g_grids;
 
-template <typename K>
-uint32_t grid_for(K kernel, int block, int sms) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
-  return (uint32_t)(per_sm * sms);
+// Threads per block of k_extend and k_connect.
+uint32_t trace_block(const WaveOptions& opt) {
+  return opt.trace_block == 64 || opt.trace_block == 256 ? opt.trace_block : (uint32_t)kTraceBlock;
 }
 
 // Surface (no media, no adjoint) extend and shade launches for scene
@@ -691,13 +691,34 @@ void prepare_persistent_grids() {
   g_grids = g;
 }
 
+void launch_connect(const ShadowQueue& q, uint32_t turn, const JobDesc* jobs, WaveCounters* counters,
+                    const WaveOptions& opt, cudaStream_t stream) {
+  ShadowQueue Q = q;
+  Q.turn = turn;
+  const uint32_t tb = trace_block(opt);
+  const uint32_t grid = g_grids.connect[tb == 64 ? 0 : (tb == 128 ? 1 : 2)];
+  if (opt.features & kFeatSpheres)
+    k_connect<kFeatSpheres><<<grid, tb, occluded_shared_bytes(tb), stream>>>(Q, jobs, counters);
+  else
+    k_connect<0><<<grid, tb, occluded_shared_bytes(tb), stream>>>(Q, jobs, counters);
+}
+
 uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, WaveControl* ctl, const JobDesc* jobs,
                      uint32_t n_jobs, WaveCounters* counters, const WaveOptions& opt, cudaEvent_t* ev,
-                     cudaStream_t stream, unsigned long long graph_condition) {
+                     cudaStream_t stream, unsigned long long graph_condition, const WaveFork* fork) {
   prepare_persistent_grids();
-  const PersistentGrids& g = g_grids;
   const bool adjoint = opt.adjoint;
-  const ShadowQueue* defer = (!opt.volumes && opt.defer_shadows && !adjoint) ? &opt.shadow_queue : nullptr;
+  const bool defers = defers_shadows(opt);
+  const uint32_t turn = fork ? fork->turn : 0u;
+  ShadowQueue queue = opt.shadow_queue;
+  queue.turn = turn;
+  const ShadowQueue* defer = defers ? &queue : nullptr;
+  if (fork) {
+    cudaEventRecord(fork->begin, stream);
+    cudaStreamWaitEvent(fork->stream, fork->begin);
+    launch_connect(opt.shadow_queue, turn ^ 1u, jobs, counters, opt, fork->stream);
+    cudaEventRecord(fork->end, fork->stream);
+  }
   const bool sort_hits = opt.sort_hits;
   HitPool Hs = H;
   if (!sort_hits) Hs.order = nullptr;
@@ -709,7 +730,7 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
   const uint32_t blocks_256 = (cap + 255) / 256, blocks_trace = (cap + kTraceBlock - 1) / kTraceBlock;
   // continuing rays grouped before tracing (the pool must have the key arrays)
   const bool sort_rays = opt.sort_rays && H.ray_key && H.ray_bins && H.ray_order;
-  k_plan<<<1, 128, 0, stream>>>(ctl, counters);
+  k_plan<<<1, 128, 0, stream>>>(ctl, counters, turn);
   if (sort_rays) {
     // (the counts are zero: cleared when allocated, at the start of every
     // frame and by each wave's k_ray_scan_blocks)
@@ -721,7 +742,7 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
   if (ev) cudaEventRecord(ev[0], stream);
   k_generate<<<blocks_256, 256, 0, stream>>>(A, ctl, jobs, n_jobs);
   if (ev) cudaEventRecord(ev[1], stream);
-  const uint32_t tb = (opt.trace_block == 64 || opt.trace_block == 256) ? opt.trace_block : (uint32_t)kTraceBlock;
+  const uint32_t tb = trace_block(opt);
   const WaveArgs w{A, B, Hs, ctl, jobs, counters, blocks_trace, stream, tb, (cap + tb - 1) / tb,
                    sort_rays ? H.ray_order : nullptr};
   if (adjoint && opt.volumes) {
@@ -738,6 +759,7 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
   if (ev) cudaEventRecord(ev[2], stream);
   if (sort_hits) k_sort_hits<<<blocks_256, 256, 0, stream>>>(ctl, Hs, A, jobs, counters, w.ray_order);
   if (ev) cudaEventRecord(ev[3], stream);
+  if (fork) cudaStreamWaitEvent(stream, fork->end);
   if (adjoint) {
     launch_adjoint_shade(opt.volumes, feat, w, opt);
   } else if (opt.volumes) {
@@ -751,11 +773,7 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
     }
   }
   if (ev) cudaEventRecord(ev[4], stream);
-  const uint32_t conn_grid = g.connect[tb == 64 ? 0 : (tb == 128 ? 1 : 2)];
-  if (defer && (feat & kFeatSpheres))
-    k_connect<kFeatSpheres><<<conn_grid, tb, occluded_shared_bytes(tb), stream>>>(*defer, jobs, counters);
-  else if (defer)
-    k_connect<0><<<conn_grid, tb, occluded_shared_bytes(tb), stream>>>(*defer, jobs, counters);
+  if (defers && !fork) launch_connect(queue, turn, jobs, counters, opt, stream);
   if (ev) cudaEventRecord(ev[5], stream);
   k_finish<<<1, 32, 0, stream>>>(ctl, counters, graph_condition);
   return 5u + (sort_hits ? 1u : 0u) + (defer ? 1u : 0u) + (sort_rays ? 4u : 0u);

@@ -869,7 +869,7 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
         if constexpr (kDefer) {
           // the light-selection pdf enters as a factor here and as a quotient for distant lights
           if (ok) {
-            const ShadowEmit em{shadow_q, &counters->shadow_count, errors, pf.x, job, P.path_id[i], tp * inv_spp};
+            const ShadowEmit em{shadow_q, &counters->shadow_count[shadow_q.turn], errors, pf.x, job, P.path_id[i], tp * inv_spp};
             const float mul = distant ? 1.0f : safe_rcp(L.select_pdf), div = distant ? L.select_pdf : 1.0f;
             emit_shadow_ray(em, so, normalize(q.dir), maxd, ((mis * vec3(1.0f) * fc * Lc) * mul) / div);
           }
@@ -1046,7 +1046,7 @@ __global__ void __launch_bounds__(kMaxTraceBlock, kConnectBlocksPerSm * kTraceBl
   OccStack st;
   st.bind(s_occ);
   OccWalk w;
-  const uint32_t n = min(counters->shadow_count, Q.capacity);
+  const uint32_t n = min(counters->shadow_count[Q.turn], Q.capacity);
   const int lane = threadIdx.x & 31;
   uint32_t ray = kEmpty;   // queue index of this lane's ray (kEmpty: idle)
   bool exhausted = false;  // the queue has been handed out (warp-uniform)
@@ -1057,7 +1057,7 @@ __global__ void __launch_bounds__(kMaxTraceBlock, kConnectBlocksPerSm * kTraceBl
       if (idle) {
         const int leader = __ffs(idle) - 1;
         uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(&counters->shadow_cursor, (uint32_t)__popc(idle));
+        if (lane == leader) base = atomicAdd(&counters->shadow_cursor[Q.turn], (uint32_t)__popc(idle));
         base = __shfl_sync(0xFFFFFFFFu, base, leader);
         if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
         if (ray == kEmpty) {
