@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) k_sort_hits(const WaveControl* __restrict
                                                    const uint32_t* __restrict__ ray_order) {
   __shared__ uint32_t s_start[kShadeBuckets];
   const uint32_t count = ctl->count;
-  const uint32_t live = ray_order ? ctl->live : 0u;
+  const uint32_t live = ray_order ? grouped_rays(ctl) : 0u;
   if (blockIdx.x * blockDim.x >= count) return;  // (uniform per block)
   if (threadIdx.x == 0) {
     uint32_t acc = 0;
@@ -530,7 +530,7 @@ __device__ __forceinline__ uint32_t ray_group_key(const DeviceScene& S, float4 o
 
 __global__ void __launch_bounds__(256) k_ray_hist(PathPool P, const WaveControl* __restrict__ ctl, HitPool H,
                                                   const JobDesc* __restrict__ jobs) {
-  const uint32_t live = ctl->live;
+  const uint32_t live = grouped_rays(ctl);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < live; i += gridDim.x * blockDim.x) {
     const uint2 pf = P.pixel_flags[i];
     const uint32_t key = ray_group_key(c_scenes[jobs[pf.y >> kFlagJobShift].scene_slot], P.ray_o[i], P.ray_d[i]);
@@ -567,7 +567,8 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
   return x - v + (warp > 0 ? s_warp[warp - 1] : 0u);
 }
 
-__global__ void __launch_bounds__(1024) k_ray_scan_blocks(HitPool H) {
+__global__ void __launch_bounds__(1024) k_ray_scan_blocks(const WaveControl* __restrict__ ctl, HitPool H) {
+  if (grouped_rays(ctl) == 0) return;
   const uint32_t k = blockIdx.x * 1024u + threadIdx.x;
   const uint32_t v = k < kRayBins ? H.ray_bins[k] : 0u;
   uint32_t total;
@@ -579,7 +580,8 @@ __global__ void __launch_bounds__(1024) k_ray_scan_blocks(HitPool H) {
   if (threadIdx.x == 0) H.ray_bins[2 * kRayBins + blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(1024) k_ray_scan_partials(HitPool H) {
+__global__ void __launch_bounds__(1024) k_ray_scan_partials(const WaveControl* __restrict__ ctl, HitPool H) {
+  if (grouped_rays(ctl) == 0) return;
   const uint32_t k = threadIdx.x;
   const uint32_t v = k < kRayScanBlocks ? H.ray_bins[2 * kRayBins + k] : 0u;
   uint32_t total;
@@ -588,7 +590,7 @@ __global__ void __launch_bounds__(1024) k_ray_scan_partials(HitPool H) {
 }
 
 __global__ void __launch_bounds__(256) k_ray_scatter(const WaveControl* __restrict__ ctl, HitPool H) {
-  const uint32_t live = ctl->live;
+  const uint32_t live = grouped_rays(ctl);
   for (uint32_t warp_base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); warp_base < live;
        warp_base += gridDim.x * blockDim.x) {
     const uint32_t i = warp_base + (threadIdx.x & 31u);
@@ -735,8 +737,8 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
     // (the counts are zero: cleared when allocated, at the start of every
     // frame and by each wave's k_ray_scan_blocks)
     k_ray_hist<<<blocks_256, 256, 0, stream>>>(A, ctl, H, jobs);
-    k_ray_scan_blocks<<<kRayScanBlocks, 1024, 0, stream>>>(H);
-    k_ray_scan_partials<<<1, 1024, 0, stream>>>(H);
+    k_ray_scan_blocks<<<kRayScanBlocks, 1024, 0, stream>>>(ctl, H);
+    k_ray_scan_partials<<<1, 1024, 0, stream>>>(ctl, H);
     k_ray_scatter<<<blocks_256, 256, 0, stream>>>(ctl, H);
   }
   if (ev) cudaEventRecord(ev[0], stream);

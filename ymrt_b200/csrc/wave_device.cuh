@@ -95,6 +95,11 @@ __device__ __forceinline__ void generate_path(const PathPool& P, uint32_t base, 
                                               unsigned long long path_cursor, const JobDesc* __restrict__ jobs,
                                               uint32_t n_jobs);
 
+// The wave's continuing rays, when there are enough of them to be grouped (else 0).
+__device__ __forceinline__ uint32_t grouped_rays(const WaveControl* ctl) {
+  return ctl->live >= kMinGroupedRays ? ctl->live : 0u;
+}
+
 // -------------------------------------------------------------- extend ---
 
 // Counts this lane's hit under its shading bucket (kBucketNone: no hit), one
@@ -140,7 +145,7 @@ __global__ void __launch_bounds__(kMaxTraceBlock, 4 * kTraceBlock / kMaxTraceBlo
                                                            const uint32_t* __restrict__ ray_order = nullptr) {
   YM_TRAVERSAL_SHARED_DYNAMIC(s_stack);
   const uint32_t count = ctl->count;
-  const uint32_t live = ray_order ? ctl->live : 0u;
+  const uint32_t live = ray_order ? grouped_rays(ctl) : 0u;
   uint32_t tests = 0, nodes = 0, n_rays = 0;
   bool overflow = false;
   for (uint32_t warp_base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); warp_base < count;
