@@ -974,7 +974,7 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
         (uintptr_t)M.pool[0].ray_o, (uintptr_t)M.pool[1].ray_o, (uintptr_t)M.hits.bary_t, (uintptr_t)M.ctl,
         (uintptr_t)M.jobs, (uintptr_t)M.counters, (uintptr_t)jobs.size(), (uintptr_t)o.volumes,
         (uintptr_t)o.sort_hits, (uintptr_t)o.defer_shadows, (uintptr_t)o.shadow_queue.o, M.capacity,
-        (uintptr_t)o.trace_block, (uintptr_t)o.sort_rays,
+        (uintptr_t)o.trace_block, (uintptr_t)o.sort_rays, (uintptr_t)o.scene_bits,
         (uintptr_t)o.features, (uintptr_t)o.grid_grads, (uintptr_t)o.grid_tex,
         (uintptr_t)o.adjoint, (uintptr_t)o.grads, o.grad_materials};
     if (ctx->graph_key != key) {
@@ -1121,6 +1121,13 @@ uint32_t batch_features(const DeviceScene* scenes, size_t n) {
   return f;
 }
 
+// Bits that tell n scenes apart (n <= kMaxSceneSlots: at most 6).
+uint32_t scene_bits(size_t n) {
+  uint32_t bits = 0;
+  while ((size_t(1) << bits) < n) ++bits;
+  return bits;
+}
+
 // Wave options for a batch: media kernels when any job scatters in media;
 // shadow rays deferred unless a job clamps indirect light.
 int batch_options(ymrt_context* ctx, const std::vector<JobDesc>& jobs, WaveOptions* opt) {
@@ -1252,6 +1259,7 @@ int ymrt_render_batch(ymrt_context* ctx, const ymrt_job* jobs_in, int n_jobs, ym
     WaveOptions opt;
     if ((rc = batch_options(ctx, jobs, &opt)) != YMRT_OK) return rc;
     opt.features = batch_features(slots.data(), slots.size());
+    opt.scene_bits = scene_bits(slots.size());
     SlotLease lease(ctx, (uint32_t)slots.size());
     if (!lease.ok()) return ctx->fail(YMRT_ERR_INVALID, "no constant-memory scene slots for this device");
     for (JobDesc& j : jobs) j.scene_slot = lease.slot(j.scene_slot);
@@ -1333,6 +1341,7 @@ int ymrt_render_backward_ex(ymrt_context* ctx, const ymrt_job* jobs_in, int n_jo
   opt.trace_block = ctx->trace_block;
   opt.sort_rays = ctx->sort_rays;
   opt.features = batch_features(slots.data(), slots.size());
+  opt.scene_bits = scene_bits(slots.size());
   opt.grads = materials ? tg->material_grads_device : nullptr;
   opt.grad_materials = materials ? tg->n_materials : 0;
   opt.grid_grads = grid ? tg->grid_grads_device : nullptr;

@@ -478,8 +478,8 @@ __global__ void k_plan(WaveControl* ctl, WaveCounters* counters, uint32_t turn) 
 // k_shade writes them in shading order (grouped by material). Traced in that
 // order, the 32 lanes of a warp walk unrelated parts of the BVH. Before the
 // closest-hit stage, the wave's continuing slots are grouped by a key of the
-// ray's origin cell (an 8x8x8 grid over the scene's top-level bounds, Morton
-// order) and its direction (cube face and quadrant, 24 values) with one
+// ray's origin cell (a 16x16x16 grid over the scene's top-level bounds, Morton
+// order) and its direction (cube face and square of it, 96 values) with one
 // counting sort (k_ray_hist, k_ray_scan_*, k_ray_scatter), and k_extend takes
 // them in that order. The hits are written to the rays' own slots, so nothing
 // after the closest-hit stage sees the order.
@@ -495,7 +495,8 @@ __device__ __forceinline__ uint32_t face_square(float u, float major) {  // u / 
   return f > 0.0f ? min((uint32_t)f, kRayDirSplit - 1u) : 0u;
 }
 
-__device__ __forceinline__ uint32_t ray_group_key(const DeviceScene& S, float4 o, float4 d) {
+__device__ __forceinline__ uint32_t ray_group_key(uint32_t slot, uint32_t scene_bits, float4 o, float4 d) {
+  const DeviceScene& S = c_scenes[slot];
   // the scene's bounds: the top-level root's grid, origin + [0, 255] * 2^e
   const uint4 w0 = __ldg(reinterpret_cast<const uint4*>(S.tlas_nodes));
   const float lo[3] = {__uint_as_float(w0.x), __uint_as_float(w0.y), __uint_as_float(w0.z)};
@@ -509,7 +510,13 @@ __device__ __forceinline__ uint32_t ray_group_key(const DeviceScene& S, float4 o
     const float f = (p[a] - lo[a]) / ext[a] * kCells;
     cell[a] = f > 0.0f ? min((uint32_t)f, (1u << kRayCellBits) - 1u) : 0u;
   }
-  const uint32_t morton = spread3(cell[0]) | (spread3(cell[1]) << 1) | (spread3(cell[2]) << 2);
+  uint32_t morton = spread3(cell[0]) | (spread3(cell[1]) << 1) | (spread3(cell[2]) << 2);
+  // a batch of several scenes: the scene's slot in the upper bits, in the
+  // place of the cell's lowest ones. A warp of mixed scenes replays each read
+  // of a scene field from constant memory once per scene and spreads over as
+  // many geometries and permutation tables (48 previews 38.6 -> 23.9 ms, their
+  // shading 21.5 -> 8.1 ms).
+  morton = ((slot & ((1u << scene_bits) - 1u)) << (3 * kRayCellBits - scene_bits)) | (morton >> scene_bits);
   const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   uint32_t face, su, sv;
   if (ax >= ay && ax >= az) {
@@ -529,11 +536,11 @@ __device__ __forceinline__ uint32_t ray_group_key(const DeviceScene& S, float4 o
 }
 
 __global__ void __launch_bounds__(256) k_ray_hist(PathPool P, const WaveControl* __restrict__ ctl, HitPool H,
-                                                  const JobDesc* __restrict__ jobs) {
+                                                  const JobDesc* __restrict__ jobs, uint32_t scene_bits) {
   const uint32_t live = grouped_rays(ctl);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < live; i += gridDim.x * blockDim.x) {
     const uint2 pf = P.pixel_flags[i];
-    const uint32_t key = ray_group_key(c_scenes[jobs[pf.y >> kFlagJobShift].scene_slot], P.ray_o[i], P.ray_d[i]);
+    const uint32_t key = ray_group_key(jobs[pf.y >> kFlagJobShift].scene_slot, scene_bits, P.ray_o[i], P.ray_d[i]);
     H.ray_key[i] = key;
     atomicAdd(&H.ray_bins[key], 1u);
   }
@@ -736,7 +743,7 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
   if (sort_rays) {
     // (the counts are zero: cleared when allocated, at the start of every
     // frame and by each wave's k_ray_scan_blocks)
-    k_ray_hist<<<blocks_256, 256, 0, stream>>>(A, ctl, H, jobs);
+    k_ray_hist<<<blocks_256, 256, 0, stream>>>(A, ctl, H, jobs, opt.scene_bits);
     k_ray_scan_blocks<<<kRayScanBlocks, 1024, 0, stream>>>(ctl, H);
     k_ray_scan_partials<<<1, 1024, 0, stream>>>(ctl, H);
     k_ray_scatter<<<blocks_256, 256, 0, stream>>>(ctl, H);
