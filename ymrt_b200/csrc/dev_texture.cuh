@@ -18,8 +18,10 @@ namespace ym {
 
 // Lattice permutation of the reference's Perlin noise (src/TextureEval.cuh:19);
 // kept identical so that procedural densities match the reference's value for
-// value. Indexed modulo 256 (the reference stores it twice in a row).
-static __constant__ uint8_t c_perlin_perm[256] = {
+// value. Indexed modulo 256 (the reference stores it twice in a row). In
+// global memory (L1): the lanes of a warp look up different entries, which a
+// constant-bank read would replay one by one.
+static __device__ const uint8_t g_perlin_perm[256] = {
     172, 142, 240, 182, 179, 214,  29, 111, 156,   3, 131, 161, 164, 194, 243, 124,
     127, 236,  88, 166,  83, 134,  71, 183, 227, 235, 106, 226, 216,  99, 149, 241,
     206,  63,  48,  31,  20, 171,  46, 185,   6, 125, 184, 133, 199, 201,  58,  81,
@@ -39,39 +41,27 @@ static __constant__ uint8_t c_perlin_perm[256] = {
 };
 
 __device__ __forceinline__ int perlin_hash(int x, int y, int z) {
-  return c_perlin_perm[(c_perlin_perm[(c_perlin_perm[x] + y) & 255] + z) & 255];
+  return __ldg(g_perlin_perm + ((__ldg(g_perlin_perm + ((__ldg(g_perlin_perm + x) + y) & 255)) + z) & 255));
 }
 
-// Gradient dot products of the 16 lattice directions (PerlinNoiseEval).
+// Gradient dot products of the 16 lattice directions (PerlinNoiseEval): +-u
+// +- v with the signs in the low two bits and the axes (u, v) = (x, y) for 0-3,
+// 12 and 13, (x, z) for 4-7, (y, z) for 8-11, (z, y) for 14 and 15. Selects, no
+// branches: the lanes' directions differ at every corner.
 __device__ __forceinline__ float perlin_grad(int h, float x, float y, float z) {
-  switch (h & 15) {
-    case 0: return x + y;
-    case 1: return -x + y;
-    case 2: return x - y;
-    case 3: return -x - y;
-    case 4: return x + z;
-    case 5: return -x + z;
-    case 6: return x - z;
-    case 7: return -x - z;
-    case 8: return y + z;
-    case 9: return -y + z;
-    case 10: return y - z;
-    case 11: return -y - z;
-    case 12: return y + x;
-    case 13: return -x + y;
-    case 14: return -y + z;
-    default: return -y - z;
-  }
+  h &= 15;
+  const float u = h < 8 || (h & 14) == 12 ? x : (h < 12 ? y : z);
+  const float v = h < 4 || h >= 12 ? y : z;
+  return ((h & 1) ? -u : u) + ((h & 2) ? -v : v);
 }
 
 __device__ __forceinline__ float perlin_fade(float t) { return t * t * t * (t * (t * 6.0f - 15.0f) + 10.0f); }
 
 // PerlinNoiseEval (src/TextureEval.cuh:55-132). Out of line: the solid
-// nodes, fBm and turbulence call it from a dozen sites, and one shared copy
-// keeps the texture-enabled media shading kernel, which is bound by
-// instruction fetch, within its instruction cache (the 1280x720 32-spp
-// textured frame 889 -> 745 ms; the fBm media frame 892 -> 882 ms; fBm
-// itself out of line as well gained nothing more).
+// nodes, fBm and turbulence call it from a dozen sites. With the permutation
+// in L1 instead of constant memory and the gradients selected instead of
+// switched on (the 1280x720 16-spp fBm media frame 263 -> 238 ms, the 8-spp
+// solid-texture one 70 -> 58 ms).
 static __device__ __noinline__ float perlin_noise(vec3 p) {
   int x0 = (int)floorf(p.x), y0 = (int)floorf(p.y), z0 = (int)floorf(p.z);
   const float tx = p.x - (float)x0, ty = p.y - (float)y0, tz = p.z - (float)z0;
@@ -274,6 +264,31 @@ __device__ __forceinline__ int texture_inputs(uint32_t type) {
   return (type >= kTexChecker && type <= kTexWave) ? 2 : 0;
 }
 
+// A node with no inputs to walk to, or one whose inputs are constants or
+// absent: evaluated without the walk's stack. Returns false for any other.
+__device__ __forceinline__ bool constant_input(const Texture* __restrict__ tex, uint32_t child, vec3* v) {
+  *v = vec3(0.0f);
+  if (child == kEmpty) return true;
+  const uint32_t type = tex[child].type;
+  if (type == kTexConstFloat) *v = vec3(tex[child].value);
+  else if (type == kTexConstRgb) *v = tex[child].color;
+  else return false;
+  return true;
+}
+
+// One node's value, given its inputs' (read by the solid nodes only).
+template <uint32_t kF>
+__device__ __forceinline__ vec3 texture_node(const Texture& t, vec3 in0, vec3 in1, const TexCoord& tc) {
+  if (t.type == kTexConstFloat) return vec3(t.value);
+  if (t.type == kTexConstRgb) return t.color;
+  if (t.type == kTexFbm)
+    return blend(in0, in1, perlin_fbm(t.frequency * tc.p, t.lacunarity, t.gain, t.layer_count, t.amplitude, t.offset));
+  if ((kF & kFeatGrids) && t.type == kTexGrid) return vec3(grid_eval(t, tc.p));
+  if ((kF & kFeatTextures) && texture_inputs(t.type) == 2) return solid_node(t, in0, in1, tc);
+  if ((kF & kFeatTextures) && t.type == kTexImage) return image_node(t, tc);
+  return vec3(0.0f);
+}
+
 // TextureEval (src/TextureEval.cuh:419-481): a post-order walk of the node
 // graph with an explicit stack of kTextureStack nodes, as the reference; an
 // absent input reads as black. A deeper graph (the loader rejects those)
@@ -283,6 +298,16 @@ __device__ __forceinline__ int texture_inputs(uint32_t type) {
 template <uint32_t kF = kFeatAll>
 __device__ __forceinline__ vec3 texture_eval(const Texture* __restrict__ tex, uint32_t root, const TexCoord& tc,
                                              uint32_t* errors) {
+  // most nodes in use need no walk (a solid node over two constants, an
+  // image, a grid): their inputs are at hand, and the walk's frames, indexed
+  // at run time, would live in local memory (fBm media frame 238 -> 232 ms)
+  {
+    const Texture& t = tex[root];
+    const int n_in = (kF & kFeatTextures) ? texture_inputs(t.type) : (t.type == kTexFbm ? 2 : 0);
+    vec3 in0(0.0f), in1(0.0f);
+    if (n_in == 0 || (constant_input(tex, t.child[0], &in0) && constant_input(tex, t.child[1], &in1)))
+      return texture_node<kF>(t, in0, in1, tc);
+  }
   struct Frame {
     uint32_t idx;
     int parent, slot, next;
@@ -317,21 +342,7 @@ __device__ __forceinline__ vec3 texture_eval(const Texture* __restrict__ tex, ui
       g.next = 0;
       continue;
     }
-    vec3 r(0.0f);
-    if (t.type == kTexConstFloat) {
-      r = vec3(t.value);
-    } else if (t.type == kTexConstRgb) {
-      r = t.color;
-    } else if (t.type == kTexFbm) {
-      r = blend(f.in[0], f.in[1],
-                perlin_fbm(t.frequency * tc.p, t.lacunarity, t.gain, t.layer_count, t.amplitude, t.offset));
-    } else if ((kF & kFeatGrids) && t.type == kTexGrid) {
-      r = vec3(grid_eval(t, tc.p));
-    } else if ((kF & kFeatTextures) && n_in == 2) {
-      r = solid_node(t, f.in[0], f.in[1], tc);
-    } else if ((kF & kFeatTextures) && t.type == kTexImage) {
-      r = image_node(t, tc);
-    }
+    const vec3 r = texture_node<kF>(t, f.in[0], f.in[1], tc);
     if (f.parent < 0) return r;
     Frame& par = st[f.parent];
     par.in[f.slot] = r;
