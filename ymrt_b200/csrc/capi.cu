@@ -306,7 +306,7 @@ struct ymrt_scene {
     bool prepared = false;
     int cur = 0;                             // which of the pairs below holds the current order
     DeviceBuffer inst[2], bucket[2], file_idx[2];
-    DeviceBuffer scales, items, nodes, mid, kind, left, stack, wide, prims, slots, offsets, inside, camera, counts;
+    DeviceBuffer scales, items, nodes, mid, kind, left, stack, wide, prims, slots, kinds, offsets, inside, camera, counts;
   } top;
 
   template <typename T>
@@ -769,6 +769,11 @@ int ymrt_scene_upload(ymrt_context* ctx, const ymrt_host_scene* hs, const uint32
     slots[k] = make_instance_slot(s.tlas_prims[k], inst, s.i_transforms[inst.transform_idx], s.geo_desc[inst.geometry_idx]);
   }
   UP(slots, inst_slots);
+  std::vector<uint16_t> kinds(s.tlas_nodes.size());
+  top_level_kinds(s.tlas_nodes.data(), (uint32_t)kinds.size(), s.tlas_prims.data(), s.instances.data(), kinds.data());
+  UP(kinds, tlas_kinds);
+  D.boundary_count = 0;
+  for (const Instance& inst : s.instances) D.boundary_count += inst.treat_as_boundary ? 1u : 0u;
 #undef UP
   sc->pack(halton_perm, perm_len, &D.halton_perm);
   if (e == cudaSuccess) e = sc->pack_commit();
@@ -1451,6 +1456,7 @@ int ymrt_scene_set_transforms(ymrt_scene* sc, uint32_t first, uint32_t count, co
     if (e == cudaSuccess) e = T.wide.ensure(sizeof(WideNode) * std::max<size_t>(2 * (size_t)n, 2));
     if (e == cudaSuccess) e = T.prims.ensure(sizeof(uint32_t) * n);
     if (e == cudaSuccess) e = T.slots.ensure(sizeof(InstanceSlot) * n);
+    if (e == cudaSuccess) e = T.kinds.ensure(sizeof(uint16_t) * std::max<size_t>(2 * (size_t)n, 2));
     if (e == cudaSuccess) e = T.offsets.ensure(sizeof(uint32_t) * n);
     if (e == cudaSuccess) e = T.inside.ensure(n);
     if (e == cudaSuccess) e = T.camera.ensure(sizeof(RayTransfer));
@@ -1496,6 +1502,7 @@ int ymrt_scene_set_transforms(ymrt_scene* sc, uint32_t first, uint32_t count, co
   b.wide = T.wide.as<WideNode>();
   b.prims = T.prims.as<uint32_t>();
   b.slots = T.slots.as<InstanceSlot>();
+  b.kinds = T.kinds.as<uint16_t>();
   b.lights = const_cast<ShapeLight*>(D.shape_lights);
   b.light_table = const_cast<float*>(D.shape_light_table);
   b.light_count = D.shape_light_count;
@@ -1520,6 +1527,7 @@ int ymrt_scene_set_transforms(ymrt_scene* sc, uint32_t first, uint32_t count, co
   D.tlas_nodes = T.wide.as<WideNode>();
   D.tlas_prims = T.prims.as<uint32_t>();
   D.inst_slots = T.slots.as<InstanceSlot>();
+  D.tlas_kinds = T.kinds.as<uint16_t>();
   D.camera.transfer = rt;
   return YMRT_OK;
 }

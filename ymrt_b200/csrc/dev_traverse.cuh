@@ -345,7 +345,7 @@ struct ClosestHit {
 // step() visits one node or enters one instance, so a persistent kernel can
 // advance the lanes of a warp on different rays (k_extend); trace_closest_impl
 // runs the steps to the end.
-// `volume_only`: traverse only treat_as_boundary instances (TraceVolume, :434-561).
+// kVolumeOnly: traverse only treat_as_boundary instances (TraceVolume, :434-561).
 //
 // One loop serves both levels: each step takes one entry -- a top-level node,
 // an instance to enter, or a bottom-level node of the current instance -- so
@@ -357,13 +357,13 @@ struct ClosestHit {
 // kSpheres: the scene holds sphere geometry. The walk without sphere code is a
 // separate instantiation, so scenes of meshes alone keep its register
 // allocation (the sphere branch costs the triangle loop about 5%).
-template <bool kSpheres>
+template <bool kSpheres, bool kVolumeOnly>
 struct ClosestWalk {
   uint32_t slot;
   vec3 wo, wd;
   BoxRay wray;
   uint32_t last_inst, last_tri;
-  bool skip_enabled, volume_only, hit;
+  bool skip_enabled, hit;
   float t_ray, t_upper, t_lower;
   int n_nearby;
   uint32_t next;  // the entry to visit before the stack's (kEmpty: none), its entry distance
@@ -381,7 +381,7 @@ struct ClosestWalk {
   uint32_t hit_tri, hit_w, extra_w;
 
   __device__ __forceinline__ void begin(uint32_t scene, TraversalStack& st, vec3 o, vec3 d, float tmax,
-                                        uint32_t li, uint32_t lt, bool vol_only) {
+                                        uint32_t li, uint32_t lt) {
     slot = scene;
     wo = o;
     wd = d;
@@ -389,7 +389,6 @@ struct ClosestWalk {
     last_inst = li;
     last_tri = lt;
     skip_enabled = li != kEmpty && lt != kEmpty;
-    volume_only = vol_only;
     hit = false;
     t_ray = tmax;
     t_upper = t_lower = 0.0f;
@@ -483,7 +482,7 @@ struct ClosestWalk {
       const uint32_t count = (e >> kEntryCountShift) & 3u, at = e & kEntrySlotMask;
       if (count > 1) st.push(e - (1u << kEntryCountShift), etn);
       const EnteredInstance in = enter_instance(S.inst_slots, at + count - 1, wo, wd);
-      if (volume_only && !(in.flags & kSlotBoundary)) return kWalkGoing;
+      if (kVolumeOnly && !(in.flags & kSlotBoundary)) return kWalkGoing;
       inst_idx = in.inst;
       const vec3 oo = in.o;
       od = in.d;
@@ -520,6 +519,7 @@ struct ClosestWalk {
       e = in.node_offset;  // continue with the instance's root in this step
     }
     const bool in_blas = inst_base >= 0;
+    const uint32_t node = e;
     ++*node_visits;
     float tn[8];
     uint32_t imask, cbase, pbase, meta[2];
@@ -557,19 +557,20 @@ struct ClosestWalk {
         }
       }
     }
-    next = push_children(st, in_blas ? hits & imask : hits, tn, imask, meta, cbase, pbase, &next_t);
+    uint32_t go = in_blas ? hits & imask : hits;
+    if (kVolumeOnly && !in_blas) go &= __ldg(S.tlas_kinds + node);
+    next = push_children(st, go, tn, imask, meta, cbase, pbase, &next_t);
     return kWalkGoing;
   }
 };
 
 // The whole walk of one ray (see ClosestWalk).
-template <bool kSpheres>
+template <bool kSpheres, bool kVolumeOnly>
 static __device__ __noinline__ bool trace_closest_impl(uint32_t scene, TraversalStack& st, vec3 wo, vec3 wd,
                                                        float tmax, uint32_t last_inst, uint32_t last_tri,
-                                                       bool volume_only, ClosestHit* out, uint32_t* tri_tests,
-                                                       uint32_t* node_visits) {
-  ClosestWalk<kSpheres> w;
-  w.begin(scene, st, wo, wd, tmax, last_inst, last_tri, volume_only);
+                                                       ClosestHit* out, uint32_t* tri_tests, uint32_t* node_visits) {
+  ClosestWalk<kSpheres, kVolumeOnly> w;
+  w.begin(scene, st, wo, wd, tmax, last_inst, last_tri);
   while (w.step(st, out, tri_tests, node_visits) == kWalkGoing) {
   }
   return w.hit;
@@ -579,13 +580,11 @@ static __device__ __noinline__ bool trace_closest_impl(uint32_t scene, Traversal
 // `scene` (see trace_closest_impl). Out of line, so that its callers keep one
 // call site whichever instantiation runs.
 static __device__ __noinline__ bool trace_closest(uint32_t scene, TraversalStack& st, vec3 wo, vec3 wd, float tmax,
-                                              uint32_t last_inst, uint32_t last_tri, bool volume_only,
-                                              ClosestHit* out, uint32_t* tri_tests, uint32_t* node_visits) {
+                                              uint32_t last_inst, uint32_t last_tri, ClosestHit* out,
+                                              uint32_t* tri_tests, uint32_t* node_visits) {
   if (c_scenes[scene].sphere_count != 0)
-    return trace_closest_impl<true>(scene, st, wo, wd, tmax, last_inst, last_tri, volume_only, out, tri_tests,
-                                    node_visits);
-  return trace_closest_impl<false>(scene, st, wo, wd, tmax, last_inst, last_tri, volume_only, out, tri_tests,
-                                   node_visits);
+    return trace_closest_impl<true, false>(scene, st, wo, wd, tmax, last_inst, last_tri, out, tri_tests, node_visits);
+  return trace_closest_impl<false, false>(scene, st, wo, wd, tmax, last_inst, last_tri, out, tri_tests, node_visits);
 }
 
 // ------------------------------------------------ resumable occlusion walk ---
@@ -703,6 +702,7 @@ __device__ __forceinline__ int occluded_step(OccWalk& w, Stack& st, uint32_t* tr
     }
   }
   uint32_t go = in_blas ? hits & imask : hits;
+  if (!in_blas && S.boundary_count != 0) go &= __ldg(S.tlas_kinds + e) >> 8;
   while (go) {
     const int c = __ffs(go) - 1;
     go &= go - 1;

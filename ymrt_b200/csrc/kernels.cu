@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_debug_trace(uint32_t slot, int 
   ClosestHit ch;
   uint32_t tests = 0, nodes = 0;
   const bool hit = trace_closest(slot, st, o, d, kTMax, last_hit ? last_hit[2 * i] : kEmpty,
-                                 last_hit ? last_hit[2 * i + 1] : kEmpty, false, &ch, &tests, &nodes);
+                                 last_hit ? last_hit[2 * i + 1] : kEmpty, &ch, &tests, &nodes);
   inst[i] = hit ? ch.inst : kEmpty;
   tri[i] = hit ? ch.tri : kEmpty;
   t[i] = hit ? ch.t : kTMax;
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_editor_view(int slot, int width
   bool done = false;
   for (int pass = 0; pass <= kEditorPassThroughs && !done; ++pass) {
     ClosestHit ch;
-    if (!trace_closest(slot, st, o, d, kTMax, last_inst, last_tri, false, &ch, &tests, &nodes)) {
+    if (!trace_closest(slot, st, o, d, kTMax, last_inst, last_tri, &ch, &tests, &nodes)) {
       col = env_light ? background(d) : vec3(0.0f);
       done = true;
       break;

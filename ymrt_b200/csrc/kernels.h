@@ -285,6 +285,7 @@ struct TlasBuild {
   // outputs
   WideNode* wide;         // top-level nodes (at most 2n)
   uint32_t* prims;        // n: instance per top-level leaf slot
+  uint16_t* kinds;        // per top-level node: top_level_kinds
   InstanceSlot* slots;    // n: the same slots' instances for the traversal
   ShapeLight* lights;
   float* light_table;

@@ -230,6 +230,11 @@ __global__ void __launch_bounds__(kCameraThreads) k_camera_inside(TlasBuild b, v
   if (threadIdx.x == 0) b.inside[i] = (any_fwd && any_bwd) ? 1 : 0;
 }
 
+__global__ void k_tlas_kinds(TlasBuild b) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  top_level_kinds(b.wide, b.counts[0], b.prims, b.instances_out, b.kinds);
+}
+
 // The traversal's record of each top-level leaf slot (after the reorder).
 __global__ void k_instance_slots(TlasBuild b) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -273,6 +278,7 @@ void launch_tlas_rebuild(const TlasBuild& b, uint32_t max_leaf, vec3 cam_pos, ve
   k_tlas_wide<<<1, 32, 0, stream>>>(b, max_leaf);
   k_tlas_reorder<<<blocks, 128, 0, stream>>>(b);
   k_instance_slots<<<blocks, 128, 0, stream>>>(b);
+  k_tlas_kinds<<<1, 32, 0, stream>>>(b);
   k_light_count<<<blocks, 128, 0, stream>>>(b);
   k_light_offsets<<<1, 32, 0, stream>>>(b);
   k_light_fill<<<blocks, 128, 0, stream>>>(b);

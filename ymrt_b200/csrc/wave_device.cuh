@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kMaxTraceBlock, 4 * kTraceBlock / kMaxTraceBlo
     TraversalStack st;
     st.bind(s_stack);
     ClosestHit ch;
-    bool hit = trace_closest_impl<(kF & kFeatSpheres) != 0>(slot, st, o, d, kTMax, lh.x, lh.y, false, &ch, &tests, &nodes);
+    bool hit = trace_closest_impl<(kF & kFeatSpheres) != 0, false>(slot, st, o, d, kTMax, lh.x, lh.y, &ch, &tests, &nodes);
     overflow = overflow || st.overflow;
     bool volume_hit = false;
     vec3 vol_pos(0.0f);
@@ -373,7 +373,7 @@ __device__ __noinline__ vec3 trace_tr(uint32_t scene, TraversalStack& st, vec3 o
       break;
     }
     ClosestHit ch;
-    const bool hit = trace_closest_impl<(kF & kFeatSpheres) != 0>(scene, st, o, d, ray_t, last_inst, last_tri, true, &ch, tests, nodes);
+    const bool hit = trace_closest_impl<(kF & kFeatSpheres) != 0, true>(scene, st, o, d, ray_t, last_inst, last_tri, &ch, tests, nodes);
     tr *= eval_tr<kF, kAdj>(S, o, d, rt, hit ? ch.t : gmax(max_d - traced, 0.0f), hs, errors, am);
     if (!hit) break;
     traced += ch.t;
