@@ -76,18 +76,41 @@ struct ymrt_context {
   WaveCounters* counters_host = nullptr;  // pinned
   WaveControl* ctl_host = nullptr;        // pinned
   DeviceBuffer ctl_buf;
-  // CUDA graph of the wave loop (a while-loop node around two waves), cached
-  // for the memory and options it was captured with
+  // CUDA graphs of the wave loop (a while-loop node around two waves), kept
+  // for the memory, options and grid sizes they were captured with, the last
+  // used first: a program that alternates two or three kinds of call (a forward
+  // and a backward pass, previews and finals) captures each once.
   bool graph_loop = true;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t graph_exec = nullptr;
-  std::vector<uintptr_t> graph_key;
+  struct WaveGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    std::vector<uintptr_t> key;
+  };
+  static constexpr size_t kMaxGraphs = 6;
+  std::vector<WaveGraph> graphs;
+  static void destroy_graph(WaveGraph& w) {
+    if (w.exec) cudaGraphExecDestroy(w.exec);
+    if (w.graph) cudaGraphDestroy(w.graph);
+  }
   void drop_graph() {
-    if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    if (graph) cudaGraphDestroy(graph);
-    graph_exec = nullptr;
-    graph = nullptr;
-    graph_key.clear();
+    for (WaveGraph& w : graphs) destroy_graph(w);
+    graphs.clear();
+  }
+  // The graph captured with `key`, now first in the list (null: none).
+  WaveGraph* find_graph(const std::vector<uintptr_t>& key) {
+    for (size_t k = 0; k < graphs.size(); ++k)
+      if (graphs[k].key == key) {
+        std::rotate(graphs.begin(), graphs.begin() + k, graphs.begin() + k + 1);
+        return &graphs.front();
+      }
+    return nullptr;
+  }
+  void keep_graph(WaveGraph&& w) {
+    if (graphs.size() >= kMaxGraphs) {
+      destroy_graph(graphs.back());
+      graphs.pop_back();
+    }
+    graphs.insert(graphs.begin(), std::move(w));
   }
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   // the branch of the captured wave loop that traces deferred shadow rays
@@ -943,6 +966,8 @@ std::vector<DeviceScene> assign_slots(std::vector<JobDesc>& jobs, const std::vec
 // once and reused while memory and options stay the same), or, with
 // per-kernel profiling or graph_loop off, launches wave after wave and reads
 // the loop condition after each. The job images must be zeroed by the caller.
+// Returns after the stream is synchronised, with the batch's counters in
+// counters_host.
 int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& jobs, const WaveOptions& opt,
               bool profiling, bool use_graph, BatchResult* r) {
   cudaStream_t st = ctx->stream;
@@ -967,7 +992,12 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
   if ((e = cudaMemcpyAsync(M.ctl, &c, sizeof(c), cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return ctx->cuda_fail(e, "uploading the wave control");
   WaveOptions o = opt;
-  o.capacity = M.capacity;
+  // Grids for the paths there are: a wave never holds more than the batch. A
+  // power of two, so that renders of similar sizes share a captured loop (a
+  // 64x64 1-spp frame, 2^12 paths in a pool of 2^21, 0.71 -> 0.60 ms of device time).
+  o.capacity = 1024;
+  while (o.capacity < M.capacity && o.capacity < total) o.capacity *= 2;
+  o.capacity = std::min(o.capacity, M.capacity);
   if ((e = cudaMemsetAsync(M.counters, 0, sizeof(WaveCounters), st)) != cudaSuccess)
     return ctx->cuda_fail(e, "clearing the wave counters");
   if (M.hits.ray_bins && (e = cudaMemsetAsync(M.hits.ray_bins, 0, kRayBins * sizeof(uint32_t), st)) != cudaSuccess)
@@ -978,12 +1008,12 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
     const std::vector<uintptr_t> key = {
         (uintptr_t)M.pool[0].ray_o, (uintptr_t)M.pool[1].ray_o, (uintptr_t)M.hits.bary_t, (uintptr_t)M.ctl,
         (uintptr_t)M.jobs, (uintptr_t)M.counters, (uintptr_t)jobs.size(), (uintptr_t)o.volumes,
-        (uintptr_t)o.sort_hits, (uintptr_t)o.defer_shadows, (uintptr_t)o.shadow_queue.o, M.capacity,
+        (uintptr_t)o.sort_hits, (uintptr_t)o.defer_shadows, (uintptr_t)o.shadow_queue.o, M.capacity, o.capacity,
         (uintptr_t)o.trace_block, (uintptr_t)o.sort_rays, (uintptr_t)o.scene_bits,
         (uintptr_t)o.features, (uintptr_t)o.grid_grads, (uintptr_t)o.grid_tex,
         (uintptr_t)o.adjoint, (uintptr_t)o.grads, o.grad_materials};
-    if (ctx->graph_key != key) {
-      ctx->drop_graph();
+    ymrt_context::WaveGraph* loop = ctx->find_graph(key);
+    if (!loop) {
       cudaGraph_t g = nullptr;
       if ((e = cudaGraphCreate(&g, 0)) != cudaSuccess) return ctx->cuda_fail(e, "cudaGraphCreate");
       cudaGraphConditionalHandle cond;
@@ -1027,14 +1057,12 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
         cudaGraphDestroy(g);
         return ctx->cuda_fail(e, "capturing the wave-loop graph");
       }
-      ctx->graph = g;
-      ctx->graph_exec = exec;
-      ctx->graph_key = key;
+      ctx->keep_graph(ymrt_context::WaveGraph{g, exec, key});
+      loop = &ctx->graphs.front();
     }
-    if ((e = cudaGraphLaunch(ctx->graph_exec, st)) != cudaSuccess) return ctx->cuda_fail(e, "launching the wave loop");
+    if ((e = cudaGraphLaunch(loop->exec, st)) != cudaSuccess) return ctx->cuda_fail(e, "launching the wave loop");
     if ((e = cudaMemcpyAsync(&c, M.ctl, sizeof(c), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
       return ctx->cuda_fail(e, "reading the wave control");
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "wave loop");
     r->launches += 1;
   } else {
     int a = 0;
@@ -1056,6 +1084,9 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
     }
   }
   cudaEventRecord(ctx->ev_stop, st);
+  if ((e = cudaMemcpyAsync(ctx->counters_host, M.counters, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st)) !=
+      cudaSuccess)
+    return ctx->cuda_fail(e, "reading counters");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "frame");
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
@@ -1209,9 +1240,6 @@ int ymrt_render_tiles(ymrt_scene* sc, const ymrt_render_setting* setting, int fr
     if ((e = cudaMemcpyAsync(out_rgba, image, img_bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
       return ctx->cuda_fail(e, "copying image");
   }
-  if ((e = cudaMemcpyAsync(ctx->counters_host, M.counters, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st)) !=
-      cudaSuccess)
-    return ctx->cuda_fail(e, "reading counters");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "frame");
   return finish_batch(ctx, r, stats);
 }
@@ -1279,10 +1307,6 @@ int ymrt_render_batch(ymrt_context* ctx, const ymrt_job* jobs_in, int n_jobs, ym
     total.ms += r.ms;
     for (int q = 0; q < 5; ++q) total.stage_ms[q] += r.stage_ms[q];
     // counters are cleared per group: keep this group's totals
-    if ((e = cudaMemcpyAsync(ctx->counters_host, M.counters, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st)) !=
-        cudaSuccess)
-      return ctx->cuda_fail(e, "reading counters");
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "batch");
     total_counters_add(ctx, k0 == 0);
     k0 = k1;
   }
@@ -1364,10 +1388,6 @@ int ymrt_render_backward_ex(ymrt_context* ctx, const ymrt_job* jobs_in, int n_jo
     return ctx->cuda_fail(e, "clearing the grid gradients");
   BatchResult r;
   if ((rc = run_batch(ctx, M, jobs, opt, ctx->profiling, ctx->graph_loop, &r)) != YMRT_OK) return rc;
-  if ((e = cudaMemcpyAsync(ctx->counters_host, M.counters, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st)) !=
-      cudaSuccess)
-    return ctx->cuda_fail(e, "reading counters");
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "backward");
   return finish_batch(ctx, r, stats);
 }
 
@@ -1784,9 +1804,6 @@ int ymrt_render_tiles_noalloc(ymrt_scene* sc, const ymrt_render_setting* setting
   opt.features = batch_features(&scene, 1);
   BatchResult r;
   if ((rc = run_batch(ctx, M, jobs, opt, false, false, &r)) != YMRT_OK) return rc;
-  if ((e = cudaMemcpyAsync(ctx->counters_host, M.counters, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st)) !=
-      cudaSuccess)
-    return ctx->cuda_fail(e, "reading counters");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "frame");
   return finish_batch(ctx, r, stats);
 }
@@ -2125,9 +2142,6 @@ int ymrt_debug_record_paths(ymrt_scene* sc, const ymrt_render_setting* setting, 
   uint32_t count = 0;
   sg.back(&count, d_count, 1);
   sg.back(out_rgba, reinterpret_cast<float*>(image), 4 * (size_t)n_pixels);
-  if ((e = cudaMemcpyAsync(ctx->counters_host, M.counters, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st)) !=
-      cudaSuccess)
-    return ctx->cuda_fail(e, "reading counters");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess || sg.err != cudaSuccess)
     return ctx->cuda_fail(e != cudaSuccess ? e : sg.err, "recording paths");
   const uint32_t kept = std::min<uint32_t>(count, (uint32_t)capacity);
