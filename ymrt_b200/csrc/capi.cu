@@ -125,6 +125,8 @@ struct ymrt_context {
   bool defer_shadows = true;
   bool sort_rays = true;  // YMRT_OPT_SORT_RAYS
   DeviceBuffer shadow_buf;
+  DeviceBuffer vertex_buf;
+  VertexQueue vertices{};
   ShadowQueue shadow_queue{};
   // pinned host staging of scene uploads (grown on demand, kept)
   void* staging = nullptr;
@@ -213,6 +215,35 @@ struct ymrt_context {
     hits.bucket = reinterpret_cast<uint8_t*>(h);
     pool_capacity = capacity;
     shadow_queue = ShadowQueue{};
+    vertices = VertexQueue{};
+    return YMRT_OK;
+  }
+
+  // Vertices between the phases of adjoint shading.
+  // For `paths` paths, at most a pool of them (no wave holds more).
+  int ensure_vertices(unsigned long long paths) {
+    size_t n = 1024;
+    while (n < pool_capacity && n < paths) n *= 2;
+    n = std::min<size_t>(n, pool_capacity);
+    if (vertices.capacity >= n) return YMRT_OK;
+    const size_t words = kVertexStateWords + kVertexLobeWords + kVertexAdjointWords + kVertexPassWords + 3;
+    cudaError_t e = vertex_buf.ensure(n * (words * sizeof(uint4) + 4 * sizeof(uint32_t)));
+    if (e != cudaSuccess) return cuda_fail(e, "allocating shading vertices");
+    uint4* p = vertex_buf.as<uint4>();
+    VertexQueue X{};
+    X.state = p; p += n * kVertexStateWords;
+    X.lobes = p; p += n * kVertexLobeWords;
+    X.adjoint = p; p += n * kVertexAdjointWords;
+    X.pass = p; p += n * kVertexPassWords;
+    X.ray_o = reinterpret_cast<float4*>(p); p += n;
+    X.ray_d = reinterpret_cast<float4*>(p); p += n;
+    X.result = reinterpret_cast<float4*>(p); p += n;
+    X.flags = reinterpret_cast<uint32_t*>(p);
+    X.dim = X.flags + n;
+    X.queue = X.dim + n;
+    X.queue_tr = X.queue + n;
+    X.capacity = (uint32_t)n;
+    vertices = X;
     return YMRT_OK;
   }
 
@@ -1011,7 +1042,7 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
         (uintptr_t)o.sort_hits, (uintptr_t)o.defer_shadows, (uintptr_t)o.shadow_queue.o, M.capacity, o.capacity,
         (uintptr_t)o.trace_block, (uintptr_t)o.sort_rays, (uintptr_t)o.scene_bits,
         (uintptr_t)o.features, (uintptr_t)o.grid_grads, (uintptr_t)o.grid_tex,
-        (uintptr_t)o.adjoint, (uintptr_t)o.grads, o.grad_materials};
+        (uintptr_t)o.adjoint, (uintptr_t)o.grads, o.grad_materials, (uintptr_t)o.vertices.state, o.vertices.capacity, o.light_kinds};
     ymrt_context::WaveGraph* loop = ctx->find_graph(key);
     if (!loop) {
       cudaGraph_t g = nullptr;
@@ -1162,6 +1193,22 @@ uint32_t scene_bits(size_t n) {
   uint32_t bits = 0;
   while ((size_t(1) << bits) < n) ++bits;
   return bits;
+}
+
+// What the phases of adjoint shading need: the vertices' memory and
+// the kinds of light any job samples.
+int phase_options(ymrt_context* ctx, const std::vector<JobDesc>& jobs, WaveOptions* opt) {
+  unsigned long long paths = 0;
+  for (const JobDesc& j : jobs) paths += j.path_count;
+  int rc = ctx->ensure_vertices(paths);
+  if (rc != YMRT_OK) return rc;
+  opt->vertices = ctx->vertices;
+  opt->light_kinds = 0;
+  for (const JobDesc& j : jobs) {
+    if (j.setting.enable_distant_light) opt->light_kinds |= 1u;
+    if (j.setting.enable_shape_light) opt->light_kinds |= 2u;
+  }
+  return YMRT_OK;
 }
 
 // Wave options for a batch: media kernels when any job scatters in media;
@@ -1375,6 +1422,7 @@ int ymrt_render_backward_ex(ymrt_context* ctx, const ymrt_job* jobs_in, int n_jo
   opt.grad_materials = materials ? tg->n_materials : 0;
   opt.grid_grads = grid ? tg->grid_grads_device : nullptr;
   opt.grid_tex = grid ? tg->grid_texture : kEmpty;
+  if ((rc = phase_options(ctx, jobs, &opt)) != YMRT_OK) return rc;
   SlotLease lease(ctx, (uint32_t)slots.size());
   if (!lease.ok()) return ctx->fail(YMRT_ERR_INVALID, "no constant-memory scene slots for this device");
   for (JobDesc& j : jobs) j.scene_slot = lease.slot(j.scene_slot);

@@ -667,8 +667,8 @@ void launch_extend_surface(const WaveArgs& w) {
 template <uint32_t kF>
 void launch_shade_surface(const ShadowQueue* defer, const WaveArgs& w) {
   constexpr uint32_t kS = surface_features(kF);
-  if (defer) launch_shade<false, true, false, kS>(w, *defer);
-  else launch_shade<false, false, false, kS>(w, ShadowQueue{});
+  if (defer) launch_shade<false, true, kS>(w, *defer);
+  else launch_shade<false, false, kS>(w, ShadowQueue{});
 }
 
 }  // namespace
@@ -691,10 +691,10 @@ void prepare_persistent_grids() {
   }
   allow_trace_shared(k_extend<false, 0>);
   allow_trace_shared(k_extend<false, kFeatSpheres>);
-  allow_shade_shared<false, false, 0>();
-  allow_shade_shared<false, false, kFeatSpheres>();
-  allow_shade_shared<false, false, kFeatTextures>();
-  allow_shade_shared<false, false, kFeatSpheres | kFeatTextures>();
+  allow_shade_shared<false, 0>();
+  allow_shade_shared<false, kFeatSpheres>();
+  allow_shade_shared<false, kFeatTextures>();
+  allow_shade_shared<false, kFeatSpheres | kFeatTextures>();
   prepare_media_kernels();
   prepare_adjoint_kernels();
   g_grids = g;
@@ -769,8 +769,11 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
   if (sort_hits) k_sort_hits<<<blocks_256, 256, 0, stream>>>(ctl, Hs, A, jobs, counters, w.ray_order);
   if (ev) cudaEventRecord(ev[3], stream);
   if (fork) cudaStreamWaitEvent(stream, fork->end);
+  uint32_t shade_launches = 1;
   if (adjoint) {
-    launch_adjoint_shade(opt.volumes, feat, w, opt);
+    WaveOptions po = opt;
+    po.connect_blocks = g_grids.connect[1];
+    shade_launches = launch_adjoint_shade(opt.volumes, feat, w, po);
   } else if (opt.volumes) {
     launch_media_shade(feat, w);
   } else {
@@ -785,7 +788,7 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
   if (defers && !fork) launch_connect(queue, turn, jobs, counters, opt, stream);
   if (ev) cudaEventRecord(ev[5], stream);
   k_finish<<<1, 32, 0, stream>>>(ctl, counters, graph_condition);
-  return 5u + (sort_hits ? 1u : 0u) + (defer ? 1u : 0u) + (sort_rays ? 4u : 0u);
+  return 4u + shade_launches + (sort_hits ? 1u : 0u) + (defer ? 1u : 0u) + (sort_rays ? 4u : 0u);
 }
 
 cudaError_t read_bound_record(uint32_t* words, int n_words, bool clear, cudaStream_t stream) {

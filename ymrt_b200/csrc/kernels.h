@@ -108,10 +108,40 @@ struct ShadowQueue {
   uint32_t turn;   // which of WaveCounters' shadow counts and cursors the wave uses
 };
 
+// Vertices of one wave between the phases of k_shade (the adjoint pass), by
+// position in the wave's hit list, and the shadow rays of the
+// current pass. Words are arrays over all vertices, one after the other.
+struct VertexQueue {
+  uint32_t* flags;     // kVertex* (0: no next-event estimation at this vertex)
+  uint32_t* dim;       // the sampler's next dimension
+  uint4* state;        // 8 words: radiance + light, direct light + its pdf, then surface point, frame and lobe weights
+  uint4* lobes;        // 4 words per lobe
+  uint4* adjoint;      // 7 words: the gradients so far and the lobe derivative data
+  uint4* pass;         // 3 words: MIS weight, BSDF or phase value, radiance, direction
+  float4* ray_o;       // origin, maximum distance
+  float4* ray_d;       // direction, kRay* and the scene slot
+  float4* result;      // transmittance, 1 when the ray reached the light (else 0)
+  uint32_t* queue;     // vertices with a ray in this pass
+  uint32_t* queue_tr;  // those whose ray is unoccluded and crosses media
+  uint32_t capacity;
+};
+constexpr uint32_t kVertexStateWords = 8, kVertexLobeWords = 4 * 5, kVertexAdjointWords = 7, kVertexPassWords = 3;
+constexpr uint32_t kVertexSurface = 1, kVertexScatter = 2, kVertexRay = 4;  // VertexQueue::flags
+constexpr uint32_t kRayCrosses = 1, kRayMedia = 2, kRaySlotShift = 8;       // VertexQueue::ray_d.w
+// One launch of a phased k_shade: pass `phase` of `passes` (phase == passes:
+// the continuation). kinds: the light kinds a job of the batch samples (1
+// distant, 2 shape).
+struct ShadePhase {
+  VertexQueue X{};
+  int phase = 0, passes = 0;
+  uint32_t kinds = 0;
+};
+
 struct WaveCounters {
   // cleared at the start of every wave (the first kWaveClearBytes bytes)
   uint32_t next_count;             // paths written to the next pool
   uint32_t hit_count;              // hits (slots listed in HitPool::order when sorting)
+  uint32_t ray_count[4], ray_cursor[4], tr_count[4];  // VertexQueue rays per pass: queued, handed out, in media
   uint32_t bucket_count[kShadeBuckets];
   uint32_t bucket_fill[kShadeBuckets];
   // cleared by the wave that fills the queue again, one pair for each of two
@@ -214,6 +244,9 @@ struct WaveOptions {
   uint32_t scene_bits = 0;     // ceil(log2) of the batch's distinct scenes: the grouping keeps them apart
   bool defer_shadows = false;  // queue surface shadow rays for k_connect (ignored with volumes)
   uint32_t features = kFeatAll;  // scene features of the batch (kFeatSpheres | kFeatGrids | kFeatTextures)
+  VertexQueue vertices{};        // adjoint: vertices between the phases of k_shade
+  uint32_t light_kinds = 0;      // adjoint: ShadePhase::kinds
+  uint32_t connect_blocks = 0;   // (set by launch_wave) resident 128-thread blocks of k_connect and k_occlude
   ShadowQueue shadow_queue{};
   bool adjoint = false;        // path-replay adjoint pass (no deferral)
   float* grads = nullptr;      // adjoint: dLoss/dParam, kGradParams per material
@@ -245,7 +278,7 @@ void prepare_adjoint_kernels();
 void launch_media_extend(uint32_t features, const WaveArgs& w);
 void launch_media_shade(uint32_t features, const WaveArgs& w);
 void launch_adjoint_extend_media(const WaveArgs& w, const WaveOptions& opt);
-void launch_adjoint_shade(bool volumes, uint32_t features, const WaveArgs& w, const WaveOptions& opt);
+uint32_t launch_adjoint_shade(bool volumes, uint32_t features, const WaveArgs& w, const WaveOptions& opt);
 cudaError_t upload_slots_media(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, cudaStream_t stream);
 cudaError_t upload_slots_adjoint(const DeviceScene* scenes, const uint32_t* slots, uint32_t n, cudaStream_t stream);
 struct BoundRecord;

@@ -8,15 +8,6 @@
 
 namespace ym {
 
-namespace {
-
-template <uint32_t kS>
-void surface_adjoint_shade(const WaveArgs& w, const WaveOptions& opt) {
-  launch_shade<false, false, true, kS>(w, ShadowQueue{}, opt.grads, opt.grad_materials);
-}
-
-}  // namespace
-
 void launch_adjoint_extend_media(const WaveArgs& w, const WaveOptions& opt) {
   // free flight with the density-grid terms (one instantiation, all features)
   const auto k = k_extend<true, kFeatAll, true>;
@@ -24,28 +15,17 @@ void launch_adjoint_extend_media(const WaveArgs& w, const WaveOptions& opt) {
                                                                            opt.grid_grads, opt.grid_tex, w.ray_order);
 }
 
-void launch_adjoint_shade(bool volumes, uint32_t features, const WaveArgs& w, const WaveOptions& opt) {
-  if (volumes) {
-    launch_shade<true, false, true, kFeatAll>(w, ShadowQueue{}, opt.grads, opt.grad_materials, opt.grid_grads,
-                                              opt.grid_tex);
-    return;
-  }
+uint32_t launch_adjoint_shade(bool volumes, uint32_t features, const WaveArgs& w, const WaveOptions& opt) {
+  if (volumes) return launch_shade_phases<true, kFeatAll>(w, opt);
   switch (surface_features(features)) {
-    case 0: surface_adjoint_shade<0>(w, opt); break;
-    case kFeatSpheres: surface_adjoint_shade<kFeatSpheres>(w, opt); break;
-    case kFeatTextures: surface_adjoint_shade<kFeatTextures>(w, opt); break;
-    default: surface_adjoint_shade<kFeatSpheres | kFeatTextures>(w, opt); break;
+    case 0: return launch_shade_phases<false, 0>(w, opt);
+    case kFeatSpheres: return launch_shade_phases<false, kFeatSpheres>(w, opt);
+    case kFeatTextures: return launch_shade_phases<false, kFeatTextures>(w, opt);
+    default: return launch_shade_phases<false, kFeatSpheres | kFeatTextures>(w, opt);
   }
 }
 
-void prepare_adjoint_kernels() {
-  allow_trace_shared(k_extend<true, kFeatAll, true>);
-  allow_shade_shared<false, true, 0>();
-  allow_shade_shared<false, true, kFeatSpheres>();
-  allow_shade_shared<false, true, kFeatTextures>();
-  allow_shade_shared<false, true, kFeatSpheres | kFeatTextures>();
-  allow_shade_shared<true, true, kFeatAll>();
-}
+void prepare_adjoint_kernels() { allow_trace_shared(k_extend<true, kFeatAll, true>); }
 
 cudaError_t upload_slots_adjoint(const DeviceScene* scenes, const uint32_t* slots, uint32_t n,
                                  cudaStream_t stream) {

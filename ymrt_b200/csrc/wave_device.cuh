@@ -555,7 +555,7 @@ __device__ __forceinline__ void emit_shadow_ray(const ShadowEmit& em, vec3 o, ve
 // sphere) or a distant light, and the probability of the choice.
 struct ChosenLight {
   bool distant;
-  int index;        // distant: into S.distant_lights
+  int index;        // into S.distant_lights or S.shape_lights
   float area;       // shape lights
   float select_pdf;
   LightTri tri;     // shape lights
@@ -569,7 +569,17 @@ __device__ __forceinline__ void choose_light(const DeviceScene& S, bool distant,
     L.index = gmax(gmin((int)(u * S.distant_light_count), (int)S.distant_light_count - 1), 0);
     return;
   }
-  const ShapeLight sl = S.shape_lights[sample_light_power(S, u, &L.select_pdf)];
+  L.index = sample_light_power(S, u, &L.select_pdf);
+  const ShapeLight sl = S.shape_lights[L.index];
+  L.area = sl.area;
+  L.tri = load_light_tri<kF>(S, sl);
+}
+// The light of an earlier choice (L.index, L.select_pdf).
+template <uint32_t kF>
+__device__ __forceinline__ void reload_light(const DeviceScene& S, bool distant, ChosenLight& L) {
+  L.distant = distant;
+  if (distant) return;
+  const ShapeLight sl = S.shape_lights[L.index];
   L.area = sl.area;
   L.tri = load_light_tri<kF>(S, sl);
 }
@@ -628,14 +638,124 @@ constexpr uint32_t shade_blocks_per_sm() {  // 128 registers a thread
   return 512 / shade_threads<kVol, kDefer, kAdj, kF>();
 }
 
+// The coincident hits of path slot i (at least the hit itself); returns their number.
+__device__ __forceinline__ int load_nearby(const HitPool& H, uint32_t i, uint4 ids, float t, NearbyHit* nb) {
+  const int n = (int)(ids.w & 0xFFu);
+  if (ids.w & kNearbyExplicit) {
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+      const uint4 e = H.nearby[(size_t)i * kMaxNearby + k];
+      nb[k] = NearbyHit{e.x, __uint_as_float(e.y), (int)e.z};
+    }
+  } else {
+    nb[0] = NearbyHit{ids.x, t, (int)(ids.z & 1u)};
+  }
+  return n;
+}
+
+// A vertex kept between the launches of a phased k_shade: surface point and
+// shading frame in six 16-byte words, each lobe in four, word k of all
+// vertices together (a warp's accesses are contiguous).
+__device__ __forceinline__ void store_vertex(const VertexQueue& X, uint32_t t, const SurfacePoint& sp,
+                                             const LayeredBsdf& B) {
+  const size_t n = X.capacity;
+  uint4* v = X.state + 2 * n + t;
+  v[0] = make_uint4(f2u(sp.p.x), f2u(sp.p.y), f2u(sp.p.z), f2u(sp.p_err.x));
+  v[n] = make_uint4(f2u(sp.p_err.y), f2u(sp.p_err.z), f2u(sp.ng.x), f2u(sp.ng.y));
+  v[2 * n] = make_uint4(f2u(sp.ng.z), f2u(B.t.x), f2u(B.t.y), f2u(B.t.z));
+  v[3 * n] = make_uint4(f2u(B.b.x), f2u(B.b.y), f2u(B.b.z), f2u(B.n.x));
+  v[4 * n] = make_uint4(f2u(B.n.y), f2u(B.n.z), (uint32_t)B.count, f2u(B.w[0]));
+  if (B.count > 1) v[5 * n] = make_uint4(f2u(B.w[1]), f2u(B.w[2]), f2u(B.w[3]), f2u(B.w[4]));
+#pragma unroll 1
+  for (int c = 0; c < B.count; ++c) {
+    const Lobe& l = B.lobe[c];
+    uint4* q = X.lobes + (size_t)c * 4 * n + t;
+    q[0] = make_uint4((uint32_t)l.type, f2u(l.albedo.x), f2u(l.albedo.y), f2u(l.albedo.z));
+    q[n] = make_uint4(f2u(l.nt.x), f2u(l.nt.y), f2u(l.nt.z), f2u(l.ni));
+    q[2 * n] = make_uint4(f2u(l.kt.x), f2u(l.kt.y), f2u(l.kt.z), f2u(l.ax));
+    q[3 * n] = make_uint4(f2u(l.ay), (uint32_t)l.is_metal, (uint32_t)l.role, 0u);
+  }
+}
+__device__ __forceinline__ void load_vertex(const VertexQueue& X, uint32_t t, SurfacePoint& sp, LayeredBsdf& B) {
+  const size_t n = X.capacity;
+  const uint4* v = X.state + 2 * n + t;
+  const uint4 a = v[0], b = v[n], c = v[2 * n], d = v[3 * n], e = v[4 * n];
+  sp.p = vec3(u2f(a.x), u2f(a.y), u2f(a.z));
+  sp.p_err = vec3(u2f(a.w), u2f(b.x), u2f(b.y));
+  sp.ng = vec3(u2f(b.z), u2f(b.w), u2f(c.x));
+  B.t = vec3(u2f(c.y), u2f(c.z), u2f(c.w));
+  B.b = vec3(u2f(d.x), u2f(d.y), u2f(d.z));
+  B.n = vec3(u2f(d.w), u2f(e.x), u2f(e.y));
+  B.count = (int)e.z;
+  B.w[0] = u2f(e.w);
+  if (B.count > 1) {
+    const uint4 f = v[5 * n];
+    B.w[1] = u2f(f.x);
+    B.w[2] = u2f(f.y);
+    B.w[3] = u2f(f.z);
+    B.w[4] = u2f(f.w);
+  }
+#pragma unroll 1
+  for (int k = 0; k < B.count; ++k) {
+    const uint4* q = X.lobes + (size_t)k * 4 * n + t;
+    const uint4 q0 = q[0], q1 = q[n], q2 = q[2 * n], q3 = q[3 * n];
+    Lobe& l = B.lobe[k];
+    l.type = (int)q0.x;
+    l.albedo = vec3(u2f(q0.y), u2f(q0.z), u2f(q0.w));
+    l.nt = vec3(u2f(q1.x), u2f(q1.y), u2f(q1.z));
+    l.ni = u2f(q1.w);
+    l.kt = vec3(u2f(q2.x), u2f(q2.y), u2f(q2.z));
+    l.ax = u2f(q2.w);
+    l.ay = u2f(q3.x);
+    l.is_metal = (int)q3.y;
+    l.role = (int)q3.z;
+  }
+}
+// The adjoint's data of the vertex: its gradients so far, and (once) the rest.
+__device__ __forceinline__ void store_adjoint(const VertexQueue& X, uint32_t t, const AdjCtx& a, bool gradients_only) {
+  const size_t n = X.capacity;
+  uint4* v = X.adjoint + t;
+  v[0] = make_uint4(f2u(a.g[0]), f2u(a.g[1]), f2u(a.g[2]), f2u(a.g[3]));
+  if (gradients_only) return;
+  v[n] = make_uint4(f2u(a.weight.x), f2u(a.weight.y), f2u(a.weight.z), f2u(a.lambert_coeff.x));
+  v[2 * n] = make_uint4(f2u(a.lambert_coeff.y), f2u(a.lambert_coeff.z), f2u(a.metal_n[0].x), f2u(a.metal_n[0].y));
+  v[3 * n] = make_uint4(f2u(a.metal_n[0].z), f2u(a.metal_n[1].x), f2u(a.metal_n[1].y), f2u(a.metal_n[1].z));
+  v[4 * n] = make_uint4(f2u(a.metal_k[0].x), f2u(a.metal_k[0].y), f2u(a.metal_k[0].z), f2u(a.metal_k[1].x));
+  v[5 * n] = make_uint4(f2u(a.metal_k[1].y), f2u(a.metal_k[1].z), f2u(a.ax[0]), f2u(a.ax[1]));
+  v[6 * n] = make_uint4(f2u(a.ay[0]), f2u(a.ay[1]), 0u, 0u);
+}
+__device__ __forceinline__ void load_adjoint(const VertexQueue& X, uint32_t t, AdjCtx& a) {
+  static_assert(kGradParams == 4, "one 16-byte word of gradients");
+  const size_t n = X.capacity;
+  const uint4* v = X.adjoint + t;
+  const uint4 g = v[0], b = v[n], c = v[2 * n], d = v[3 * n], e = v[4 * n], f = v[5 * n], h = v[6 * n];
+  a.g[0] = u2f(g.x);
+  a.g[1] = u2f(g.y);
+  a.g[2] = u2f(g.z);
+  a.g[3] = u2f(g.w);
+  a.weight = vec3(u2f(b.x), u2f(b.y), u2f(b.z));
+  a.lambert_coeff = vec3(u2f(b.w), u2f(c.x), u2f(c.y));
+  a.metal_n[0] = vec3(u2f(c.z), u2f(c.w), u2f(d.x));
+  a.metal_n[1] = vec3(u2f(d.y), u2f(d.z), u2f(d.w));
+  a.metal_k[0] = vec3(u2f(e.x), u2f(e.y), u2f(e.z));
+  a.metal_k[1] = vec3(u2f(e.w), u2f(f.x), u2f(f.y));
+  a.ax[0] = u2f(f.z);
+  a.ax[1] = u2f(f.w);
+  a.ay[0] = u2f(h.x);
+  a.ay[1] = u2f(h.y);
+}
+
 template <bool kVol, bool kDefer, bool kAdj, uint32_t kF>
 __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade_blocks_per_sm<kVol, kDefer, kAdj, kF>()) k_shade(
     PathPool P, const WaveControl* __restrict__ ctl, HitPool H, PathPool Q, const JobDesc* __restrict__ jobs,
     WaveCounters* counters, ShadowQueue shadow_q, float* grads = nullptr, uint32_t grad_materials = 0,
-    float* grid_grads = nullptr, uint32_t grid_tex = kEmpty) {
+    ShadePhase ph = ShadePhase{}) {
   static_assert(!(kVol && kDefer), "volume transmittance needs the path's sampler: shadow rays are traced inline");
-  static_assert(!(kAdj && kDefer), "the adjoint pass traces its shadow rays inline");
+  static_assert(!(kAdj && kDefer), "the adjoint pass traces its shadow rays in turn");
   constexpr bool kSpheres = (kF & kFeatSpheres) != 0;
+  constexpr bool kPhased = kAdj;
+  const VertexQueue& X = ph.X;
+  const bool first = !kPhased || ph.phase == 0, last = !kPhased || ph.phase == ph.passes;
   float* s_grad = nullptr;
   const uint32_t n_slots = min(grad_materials, (uint32_t)kMaxGradMaterials) * kGradParams;
   if constexpr (kAdj) {
@@ -645,7 +765,7 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
     __syncthreads();
   }
   TraversalStack st;
-  if constexpr (!kDefer) {
+  if constexpr (!kDefer && !kPhased) {
     YM_TRAVERSAL_SHARED_DYNAMIC(s_stack);
     st.bind(s_stack);
   } else {
@@ -665,6 +785,12 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
     const uint32_t i = active ? (listed ? H.order[t_idx] : t_idx) : 0u;
     const uint2 pf = active ? P.pixel_flags[i] : make_uint2(kEmpty, kFlagDead);
     if (pf.y & kFlagDead) active = false;  // a miss (already accumulated) or an empty slot
+    uint32_t flags = 0u;     // (phased) kVertex*
+    if (kPhased && !first) {
+      flags = active ? X.flags[t_idx] : 0u;
+      active = flags != 0u;
+      if (!__syncthreads_or(active)) continue;
+    }
     bool alive = false;      // continues into Q
     bool ended = false;      // a path whose radiance is complete
     bool surface = false;    // a material vertex: next-event estimation and a BSDF continuation
@@ -694,7 +820,6 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
     // media of a volume vertex
     float vw[kMaxBoundaryRecord], gs[kMaxBoundaryRecord];
     int n_media = 0;
-    MediumAdj av{vec3(0.0f), grid_tex, grid_grads};
 
     if (active) {
       const float4 d4 = P.ray_d[i], t4 = P.throughput[i], r4 = P.radiance[i];
@@ -714,6 +839,7 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
       tri = ids.y;
       hit_back = (int)(ids.z & 1u);
       volume = kVol && (ids.z & 2u);
+      if (kPhased && !first) hs.dim = X.dim[t_idx];
       if (kAdj) {
         const float4 dl = J.dloss[pf.x];
         delta = vec3(dl.x, dl.y, dl.z) * inv_spp;  // dLoss/d(this path's radiance)
@@ -729,27 +855,19 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
         }
         sp.p = bary;
         inst_idx = tri = kEmpty;
-        if (kAdj) av.scale = delta * tp;  // dLoss/d(this vertex's light), before 1/select_pdf
       } else if (inst_idx == kEmpty) {
         // a miss (Ray_trace_path_tracing, src/Shading.cu:1855-1864): the
         // background when the environment light is on, then the path ends
         if (rs.enable_env_light) rad += indirect_clamp(rs, tp * background(rd), depth);
         ended = true;
       } else {
-        n_nb = (int)(ids.w & 0xFFu);
-        if (ids.w & kNearbyExplicit) {
-#pragma unroll 1
-          for (int k = 0; k < n_nb; ++k) {
-            const uint4 e = H.nearby[(size_t)i * kMaxNearby + k];
-            nb[k] = NearbyHit{e.x, __uint_as_float(e.y), (int)e.z};
-          }
-        } else {
-          nb[0] = NearbyHit{inst_idx, bt.w, hit_back};
-        }
-        sp = fetch_surface<kF>(S, inst_idx, tri, bary);
+        n_nb = load_nearby(H, i, ids, bt.w, nb);
         const Instance inst = S.instances[inst_idx];
         material = inst.material_idx;
-        if (!(material < S.material_count)) {
+        if (first) sp = fetch_surface<kF>(S, inst_idx, tri, bary);
+        if (kPhased && !first) {
+          surface = true;
+        } else if (!(material < S.material_count)) {
           ended = true;
         } else {
           const Material& mat = S.materials[material];
@@ -777,7 +895,20 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
 
     // The layered BSDF of a material vertex.
     __syncthreads();
-    if (surface) {
+    ChosenLight L;
+    vec3 direct(0.0f);
+    if (kPhased && !first && active) {
+      const uint4 m0 = X.state[t_idx], m1 = X.state[X.capacity + t_idx];
+      rad = vec3(u2f(m0.x), u2f(m0.y), u2f(m0.z));
+      direct = vec3(u2f(m1.x), u2f(m1.y), u2f(m1.z));
+      L.index = (int)m0.w;
+      L.select_pdf = u2f(m1.w);
+      if (surface) load_vertex(X, t_idx, sp, B);
+      if constexpr (kAdj) {
+        if (surface) load_adjoint(X, t_idx, adj_ctx);
+      }
+    }
+    if (first && surface) {
       const DefaultMtl& md = S.materials[material].default_mtl;
       const DefaultMtl* mp = &md;
       DefaultMtl mt;
@@ -803,6 +934,12 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
         adj_ctx.weight = delta * tp;
       }
     }
+    if constexpr (kAdj) {
+      if (!first && surface) {
+        const float4 lt = J.path_radiance[P.path_id[i]];
+        l_total = vec3(lt.x, lt.y, lt.z);
+      }
+    }
     const vec3 wo = surface ? B.to_local(-rd) : vec3(0.0f);
 
     // Next-event estimation: EvalDistantLight / EvalShapeLight (src/Shading.cu:83-198,
@@ -810,18 +947,63 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
     // (:202-291, 419-513) at volume vertices. Two kinds of light, and for each
     // a direction sampled from the light (pass 0) and one from the BSDF or the
     // phase functions (pass 1).
+    // (phased) one pass per launch: its shadow rays are queued and traced by
+    // k_occlude and k_transmit, whose answers the next launch takes up here.
+    auto kind_of = [&](int pass) { return kPhased ? (ph.kinds == 2u || pass >= 2 ? 1 : 0) : pass >> 1; };
+    auto kind_on = [&](bool distant) {
+      return (surface || (volume && n_media > 0)) &&
+             (distant ? rs.enable_distant_light && S.distant_light_count > 0
+                      : rs.enable_shape_light != 0 && S.shape_light_count > 0);
+    };
+    // a pass's contribution, and after the second of a kind the kind's estimate
+    auto finish_kind = [&](bool distant) {
+      const vec3 e = distant || (kVol && volume) ? (L.select_pdf > 0.0f ? direct / L.select_pdf : vec3(0.0f))
+                                                 : direct * safe_rcp(L.select_pdf);
+      rad += indirect_clamp(rs, tp * e, depth);
+    };
+    if constexpr (kPhased) {
+      if (!first && active) {
+        const int p = ph.phase - 1;
+        const bool distant = kind_of(p) == 0;
+        if (flags & kVertexRay) {
+          const float4 r = X.result[t_idx];
+          if (r.w != 0.0f) {
+            const uint4 p0 = X.pass[t_idx], p1 = X.pass[X.capacity + t_idx];
+            const vec3 contrib = u2f(p0.x) * vec3(r.x, r.y, r.z) * vec3(u2f(p0.y), u2f(p0.z), u2f(p0.w)) *
+                                 vec3(u2f(p1.x), u2f(p1.y), u2f(p1.z));
+            direct += contrib;
+            if constexpr (kAdj) {
+              if (surface) {
+                // d(direct)/dp = mis * tr * fc * (df/dp)/f * Lc, scaled like the estimator
+                const float mul = distant ? 1.0f : safe_rcp(L.select_pdf), div = distant ? L.select_pdf : 1.0f;
+                const uint4 p2 = X.pass[2 * (size_t)X.capacity + t_idx];
+                const vec3 dir(u2f(p1.w), u2f(p2.x), u2f(p2.y));
+                add_relative_grads(&adj_ctx, B, wo, B.to_local(dir), adj_ctx.weight * (mul / div), contrib);
+              }
+            }
+          }
+        }
+        if ((p & 1) && kind_on(distant)) finish_kind(distant);
+      }
+    }
 #pragma unroll 1
-    for (int kind = 0; kind < 2; ++kind) {
-      const bool distant = kind == 0;
-      const bool on = (surface || (volume && n_media > 0)) &&
-                      (distant ? rs.enable_distant_light && S.distant_light_count > 0
-                               : rs.enable_shape_light != 0 && S.shape_light_count > 0);
-      if (!__syncthreads_or(on)) continue;
-      ChosenLight L;
-      vec3 direct(0.0f);
-      if (on) choose_light<kF>(S, distant, hs, L);
-#pragma unroll 1
-      for (int pass = 0; pass < 2; ++pass) {
+    for (int p = kPhased ? ph.phase : 0; p < (kPhased ? min(ph.phase + 1, ph.passes) : 4); ++p) {
+      const bool distant = kind_of(p) == 0;
+      const int pass = p & 1;
+      const bool on = kind_on(distant);
+      if (!kPhased && pass == 0 && !__syncthreads_or(on)) {
+        ++p;  // neither pass of this kind
+        continue;
+      }
+      if (on) {
+        if (pass == 0) {
+          choose_light<kF>(S, distant, hs, L);
+          direct = vec3(0.0f);
+        } else if (kPhased) {
+          reload_light<kF>(S, distant, L);
+        }
+      }
+      {
         LightSample q{vec3(0.0f), vec3(0.0f), vec3(0.0f), vec3(0.0f), vec3(0.0f), 0.0f};
         vec3 f(0.0f), lwi(0.0f), so(0.0f);
         float spdf = 0.0f, maxd = kTMax;  // spdf: of the BSDF or the phase functions
@@ -879,54 +1061,59 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
             emit_shadow_ray(em, so, normalize(q.dir), maxd, ((mis * vec3(1.0f) * fc * Lc) * mul) / div);
           }
           __syncthreads();
+        } else if constexpr (kPhased) {
+          // kept for the next launch: the vertex (once), what the pass changes,
+          // and the ray
+          flags = surface || volume ? (surface ? kVertexSurface : kVertexScatter) | (ok ? kVertexRay : 0u) : 0u;
+          if (flags) {
+            if (first && surface) {
+              store_vertex(X, t_idx, sp, B);
+            }
+            if constexpr (kAdj) {
+              if (surface) store_adjoint(X, t_idx, adj_ctx, !first);
+            }
+            X.state[t_idx] = make_uint4(f2u(rad.x), f2u(rad.y), f2u(rad.z), (uint32_t)L.index);
+            X.state[X.capacity + t_idx] = make_uint4(f2u(direct.x), f2u(direct.y), f2u(direct.z), f2u(L.select_pdf));
+            X.dim[t_idx] = hs.dim;
+          }
+          if (ok) {
+            const vec3 dir = normalize(q.dir);
+            const bool media = kVol && (volume || rs.enable_volume_scattering);
+            X.ray_o[t_idx] = make_float4(so.x, so.y, so.z, maxd);
+            X.ray_d[t_idx] = make_float4(dir.x, dir.y, dir.z,
+                                         u2f(slot << kRaySlotShift | (tb ? kRayCrosses : 0u) | (media ? kRayMedia : 0u)));
+            X.pass[t_idx] = make_uint4(f2u(mis), f2u(fc.x), f2u(fc.y), f2u(fc.z));
+            X.pass[X.capacity + t_idx] = make_uint4(f2u(Lc.x), f2u(Lc.y), f2u(Lc.z), f2u(q.dir.x));
+            if (kAdj) X.pass[2 * (size_t)X.capacity + t_idx] = make_uint4(f2u(q.dir.y), f2u(q.dir.z), 0u, 0u);
+          }
+          const uint32_t at = warp_append(&counters->ray_count[p], ok);
+          if (ok) X.queue[at] = t_idx;
         } else {
           __syncthreads();
           if (ok) {
             const vec3 dir = normalize(q.dir);
             if (!trace_occluded_impl<kSpheres>(slot, st, so, dir, maxd, &tests, &nodes)) {
               vec3 tr(1.0f);
-              const PathSampler hs0 = hs;
-              const bool media = kVol && (volume || rs.enable_volume_scattering);
-              if (media) {
+              if (kVol && (volume || rs.enable_volume_scattering)) {
                 RayTransfer srt = rt;
                 if (tb) boundary_transition(S, srt, nb, n_nb, errors);
                 tr = trace_tr<kF>(slot, st, so, dir, maxd, inst_idx, tri, srt, hs, errors, &tests, &nodes);
               }
-              const vec3 contrib = mis * tr * fc * Lc;
-              direct += contrib;
-              if constexpr (kAdj) {
-                const float mul = distant || volume ? 1.0f : safe_rcp(L.select_pdf);
-                const float div = distant || volume ? L.select_pdf : 1.0f;
-                if (kVol && grid_grads && media && (!volume || L.select_pdf > 0.0f)) {
-                  // the transmittance's density-grid terms: replay its tracking with the
-                  // same samples, weighted by this ray's share of dLoss
-                  const MediumAdj am{volume ? av.scale * contrib / L.select_pdf : adj_ctx.weight * (mul / div) * contrib,
-                                     grid_tex, grid_grads};
-                  if (max_component(vabs(am.scale)) > 0.0f) {
-                    RayTransfer srt = rt;
-                    if (tb) boundary_transition(S, srt, nb, n_nb, errors);
-                    PathSampler h2 = hs0;
-                    trace_tr<kF, true>(slot, st, so, dir, maxd, inst_idx, tri, srt, h2, errors, &tests, &nodes, &am);
-                  }
-                }
-                // d(direct)/dp = mis * tr * fc * (df/dp)/f * Lc, scaled like the estimator
-                if (surface)
-                  add_relative_grads(&adj_ctx, B, wo, B.to_local(q.dir), adj_ctx.weight * (mul / div), contrib);
-              }
+              direct += mis * tr * fc * Lc;
             }
           }
           __syncthreads();
         }
       }
-      if (on) {
-        const vec3 e = distant || (kVol && volume) ? (L.select_pdf > 0.0f ? direct / L.select_pdf : vec3(0.0f))
-                                                   : direct * safe_rcp(L.select_pdf);
-        rad += indirect_clamp(rs, tp * e, depth);
-      }
+      if (!kPhased && pass == 1 && on) finish_kind(distant);
+    }
+    if (kPhased && !last) {
+      if (first && t_idx < count) X.flags[t_idx] = flags;
+      else if (active) X.flags[t_idx] = flags;
     }
 
     // The continuation: a direction from the BSDF or the phase functions.
-    if (surface || (kVol && volume)) {
+    if (last && (surface || (kVol && volume))) {
       float u0, u1, u2 = 0.0f;
       sample2d(hs, S, &u0, &u1);
       vec3 w(0.0f), wi(0.0f);
@@ -1018,21 +1205,199 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
 
 // Lets a k_shade instantiation that traces its shadow rays inline take its
 // block's traversal stacks in dynamic shared memory (more than the default 48 KB).
-template <bool kVol, bool kAdj, uint32_t kF>
+template <bool kVol, uint32_t kF>
 static void allow_shade_shared() {
-  cudaFuncSetAttribute(k_shade<kVol, false, kAdj, kF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)traversal_shared_bytes(shade_threads<kVol, false, kAdj, kF>()));
+  cudaFuncSetAttribute(k_shade<kVol, false, false, kF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)traversal_shared_bytes(shade_threads<kVol, false, false, kF>()));
 }
 
-// Launches k_shade over the wave (one thread per pool slot).
-template <bool kVol, bool kDefer, bool kAdj, uint32_t kF>
-void launch_shade(const WaveArgs& w, const ShadowQueue& q, float* grads = nullptr, uint32_t grad_materials = 0,
-                  float* grid_grads = nullptr, uint32_t grid_tex = kEmpty) {
-  constexpr uint32_t threads = shade_threads<kVol, kDefer, kAdj, kF>();
+// Launches k_shade over the wave (one thread per pool slot): the forward
+// pass, with deferred or inline shadow rays.
+template <bool kVol, bool kDefer, uint32_t kF>
+void launch_shade(const WaveArgs& w, const ShadowQueue& q) {
+  constexpr uint32_t threads = shade_threads<kVol, kDefer, false, kF>();
   const uint32_t blocks = (w.blocks * kTraceBlock + threads - 1) / threads;
   const size_t shared = kDefer ? 0 : traversal_shared_bytes(threads);
-  k_shade<kVol, kDefer, kAdj, kF><<<blocks, threads, shared, w.stream>>>(w.A, w.ctl, w.H, w.B, w.jobs, w.counters, q,
-                                                                         grads, grad_materials, grid_grads, grid_tex);
+  k_shade<kVol, kDefer, false, kF><<<blocks, threads, shared, w.stream>>>(w.A, w.ctl, w.H, w.B, w.jobs, w.counters, q);
+}
+
+// ------------------------------------------- phased next-event estimation ---
+//
+// The adjoint pass weighs each shadow ray's gradient terms by what the ray
+// finds (and with media its transmittance draws from the path's sampler), so
+// a vertex's shadow rays come one after the other. k_shade then runs in
+// phases, one per pass (light kind x estimator): it queues the pass's rays and
+// keeps the vertices; k_occlude and k_transmit trace the queue with full warps
+// over the whole GPU; the next phase takes up the answers. Traced inline, a
+// block waited at its barriers for its longest ray with a third of its lanes
+// on a ray (backward of 4 views 512x512 16 spp 67.7 -> 61.8 ms, of 4 views
+// 256x256 8 spp in fog 36.4 -> 31.4 ms). The forward media pass stays inline:
+// it gained nothing (volumetric 1280x720 227 and 227 ms, solid textures 56.8
+// inline and 58.2 phased) and would pay the extra launches in small renders.
+
+// Occlusion of a pass's queued rays: persistent, with k_connect's warp-level
+// work fetch. An unoccluded ray in media goes on to k_transmit's queue.
+template <bool kSpheres>
+static __global__ void __launch_bounds__(kTraceBlock, kConnectBlocksPerSm) k_occlude(VertexQueue X, WaveCounters* counters,
+                                                                                     int pass) {
+  extern __shared__ __align__(16) uint32_t s_occ[];  // occluded_shared_bytes(blockDim.x)
+  OccStack st;
+  st.bind(s_occ);
+  OccWalk w;
+  const uint32_t n = min(counters->ray_count[pass], X.capacity);
+  const int lane = threadIdx.x & 31;
+  uint32_t ray = kEmpty;   // the vertex whose ray this lane traces (kEmpty: idle)
+  uint32_t bits = 0;
+  bool exhausted = false;  // the queue has been handed out (warp-uniform)
+  uint32_t tests = 0, nodes = 0;
+  for (;;) {
+    if (!exhausted) {
+      const uint32_t idle = __ballot_sync(0xFFFFFFFFu, ray == kEmpty);
+      if (idle) {
+        const int leader = __ffs(idle) - 1;
+        uint32_t base = 0;
+        if (lane == leader) base = atomicAdd(&counters->ray_cursor[pass], (uint32_t)__popc(idle));
+        base = __shfl_sync(0xFFFFFFFFu, base, leader);
+        if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
+        if (ray == kEmpty) {
+          const uint32_t t = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+          if (t < n) {
+            ray = X.queue[t];
+            const float4 o = X.ray_o[ray], d = X.ray_d[ray];
+            bits = __float_as_uint(d.w);
+            w.begin(bits >> kRaySlotShift, vec3(o.x, o.y, o.z), vec3(d.x, d.y, d.z), o.w, st);
+          }
+        }
+      }
+    }
+    if (__ballot_sync(0xFFFFFFFFu, ray != kEmpty) == 0) break;
+    if (ray != kEmpty) {
+      const int r = occluded_step<kSpheres>(w, st, &tests, &nodes);
+      if (r != kWalkGoing) {
+        const bool clear = r == kWalkClear;
+        if (clear && (bits & kRayMedia)) {
+          cg::coalesced_group g = cg::coalesced_threads();
+          uint32_t base = 0;
+          if (g.thread_rank() == 0) base = atomicAdd(&counters->tr_count[pass], g.size());
+          X.queue_tr[g.shfl(base, 0) + g.thread_rank()] = ray;
+        } else {
+          X.result[ray] = clear ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        ray = kEmpty;
+      }
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    tests += __shfl_down_sync(0xFFFFFFFFu, tests, off);
+    nodes += __shfl_down_sync(0xFFFFFFFFu, nodes, off);
+  }
+  if (lane == 0) {
+    if (tests) atomicAdd(&counters->shadow_tri_tests, (unsigned long long)tests);
+    if (nodes) atomicAdd(&counters->shadow_node_visits, (unsigned long long)nodes);
+  }
+  if (st.overflow) atomicOr(&counters->errors, (uint32_t)kDevErrStack);
+}
+
+// Transmittance of a pass's unoccluded rays, from the state their vertex's
+// sampler was left in. With grid_grads, the ray's tracking is replayed with
+// the same samples for the density-grid terms, weighted by its share of dLoss.
+template <uint32_t kF>
+static __global__ void __launch_bounds__(kTraceBlock, 4) k_transmit(VertexQueue X, PathPool P, HitPool H,
+                                                                    const JobDesc* __restrict__ jobs,
+                                                                    WaveCounters* counters, int pass, bool distant,
+                                                                    float* grid_grads, uint32_t grid_tex) {
+  YM_TRAVERSAL_SHARED_DYNAMIC(s_stack);
+  TraversalStack st;
+  st.bind(s_stack);
+  const uint32_t n = min(counters->tr_count[pass], X.capacity);
+  uint32_t tests = 0, nodes = 0;
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;  // (one thread per pool slot)
+  if ((k & ~31u) >= n) return;  // (whole warps)
+  if (k < n) {
+    const uint32_t t = X.queue_tr[k];
+    const uint32_t i = H.order ? H.order[t] : t;
+    const float4 o4 = X.ray_o[t], d4 = X.ray_d[t];
+    const uint32_t bits = __float_as_uint(d4.w), slot = bits >> kRaySlotShift;
+    const vec3 o(o4.x, o4.y, o4.z), d(d4.x, d4.y, d4.z);
+    const uint4 ids = H.ids[i];
+    const bool volume = (ids.z & 2u) != 0u;
+    const uint32_t inst = volume ? kEmpty : ids.x, tri = volume ? kEmpty : ids.y;
+    RayTransfer rt;
+    rt.record_count = 0;
+    rt.max_priority_record_index = -1;
+    if (P.transfer_count[i] > 0) rt = P.transfer[i];
+    if (bits & kRayCrosses) {
+      NearbyHit nb[kMaxNearby];
+      const int n_nb = load_nearby(H, i, ids, H.bary_t[i].w, nb);
+      boundary_transition(c_scenes[slot], rt, nb, n_nb, &counters->errors);
+    }
+    const uint4 s4 = P.sampler[i];
+    PathSampler hs{(uint64_t)s4.x | ((uint64_t)s4.y << 32), X.dim[t], s4.w};
+    RayTransfer rt0;
+    const PathSampler hs0 = hs;
+    if (grid_grads) rt0 = rt;
+    const vec3 tr = trace_tr<kF>(slot, st, o, d, o4.w, inst, tri, rt, hs, &counters->errors, &tests, &nodes);
+    X.result[t] = make_float4(tr.x, tr.y, tr.z, 1.0f);
+    X.dim[t] = hs.dim;
+    if (grid_grads) {
+      const uint2 pf = P.pixel_flags[i];
+      const JobDesc& J = jobs[pf.y >> kFlagJobShift];
+      const float inv_spp = 1.0f / gmax(J.setting.ssp, 1);
+      const float4 dl = J.dloss[pf.x], t4 = P.throughput[i];
+      const vec3 weight = vec3(dl.x, dl.y, dl.z) * inv_spp * vec3(t4.x, t4.y, t4.z);
+      const uint4 p0 = X.pass[t], p1 = X.pass[X.capacity + t];
+      const vec3 contrib = u2f(p0.x) * tr * vec3(u2f(p0.y), u2f(p0.z), u2f(p0.w)) *
+                           vec3(u2f(p1.x), u2f(p1.y), u2f(p1.z));
+      const float select_pdf = u2f(X.state[X.capacity + t].w);
+      const float mul = distant ? 1.0f : safe_rcp(select_pdf), div = distant ? select_pdf : 1.0f;
+      vec3 scale(0.0f);
+      if (!volume) scale = weight * (mul / div) * contrib;
+      else if (select_pdf > 0.0f) scale = weight * contrib / select_pdf;
+      if (max_component(vabs(scale)) > 0.0f) {
+        const MediumAdj am{scale, grid_tex, grid_grads};
+        hs = hs0;
+        trace_tr<kF, true>(slot, st, o, d, o4.w, inst, tri, rt0, hs, &counters->errors, &tests, &nodes, &am);
+      }
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    tests += __shfl_down_sync(0xFFFFFFFFu, tests, off);
+    nodes += __shfl_down_sync(0xFFFFFFFFu, nodes, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (tests) atomicAdd(&counters->shadow_tri_tests, (unsigned long long)tests);
+    if (nodes) atomicAdd(&counters->shadow_node_visits, (unsigned long long)nodes);
+  }
+  if (st.overflow) atomicOr(&counters->errors, (uint32_t)kDevErrStack);
+}
+
+// A wave's adjoint shading in phases: k_shade, k_occlude and k_transmit per
+// pass, then k_shade's continuation. Returns the launches.
+template <bool kVol, uint32_t kF>
+uint32_t launch_shade_phases(const WaveArgs& w, const WaveOptions& opt) {
+  constexpr uint32_t threads = shade_threads<kVol, false, true, kF>();
+  const uint32_t blocks = (w.blocks * kTraceBlock + threads - 1) / threads;
+  ShadePhase ph;
+  ph.X = opt.vertices;
+  ph.kinds = opt.light_kinds;
+  ph.passes = ((opt.light_kinds & 1u) ? 2 : 0) + ((opt.light_kinds & 2u) ? 2 : 0);
+  uint32_t launches = 0;
+  for (ph.phase = 0; ph.phase <= ph.passes; ++ph.phase) {
+    k_shade<kVol, false, true, kF><<<blocks, threads, 0, w.stream>>>(w.A, w.ctl, w.H, w.B, w.jobs, w.counters,
+                                                                    ShadowQueue{}, opt.grads, opt.grad_materials, ph);
+    ++launches;
+    if (ph.phase == ph.passes) break;
+    k_occlude<(kF & kFeatSpheres) != 0><<<opt.connect_blocks, kTraceBlock, occluded_shared_bytes(kTraceBlock), w.stream>>>(
+        ph.X, w.counters, ph.phase);
+    ++launches;
+    if constexpr (kVol) {
+      const bool distant = ph.kinds != 2u && ph.phase < 2;
+      k_transmit<kF><<<w.blocks, kTraceBlock, traversal_shared_bytes(kTraceBlock), w.stream>>>(
+          ph.X, w.A, w.H, w.jobs, w.counters, ph.phase, distant, opt.grid_grads, opt.grid_tex);
+      ++launches;
+    }
+  }
+  return launches;
 }
 
 // ------------------------------------------------------------- connect ---

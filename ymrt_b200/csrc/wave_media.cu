@@ -18,7 +18,7 @@ void media_extend(const WaveArgs& w) {
 
 template <uint32_t kF>
 void media_shade(const WaveArgs& w) {
-  launch_shade<true, false, false, kF>(w, ShadowQueue{});
+  launch_shade<true, false, kF>(w, ShadowQueue{});
 }
 
 constexpr uint32_t kAllNodes = kFeatGrids | kFeatTextures;
@@ -48,10 +48,10 @@ void prepare_media_kernels() {
   allow_trace_shared(k_extend<true, kFeatSpheres>);
   allow_trace_shared(k_extend<true, kAllNodes>);
   allow_trace_shared(k_extend<true, kAllNodes | kFeatSpheres>);
-  allow_shade_shared<true, false, 0>();
-  allow_shade_shared<true, false, kFeatSpheres>();
-  allow_shade_shared<true, false, kAllNodes>();
-  allow_shade_shared<true, false, kAllNodes | kFeatSpheres>();
+  allow_shade_shared<true, 0>();
+  allow_shade_shared<true, kFeatSpheres>();
+  allow_shade_shared<true, kAllNodes>();
+  allow_shade_shared<true, kAllNodes | kFeatSpheres>();
 }
 
 cudaError_t upload_slots_media(const DeviceScene* scenes, const uint32_t* slots, uint32_t n,
