@@ -212,41 +212,94 @@ static __device__ __noinline__ float sampler_value(PathSampler s, uint32_t sampl
   return sobol_draw(s, table);
 }
 
+// The dimension after `dim`.
+__device__ __forceinline__ uint32_t next_dim(uint32_t dim, uint32_t sampler_type) {
+  ++dim;
+  if (sampler_type == kSamplerHalton && dim >= (uint32_t)kHaltonDims) dim = 2;
+  if (sampler_type == kSamplerSobol && dim >= 4096u) dim = 1;  // the reference wraps here (and prints a warning)
+  return dim;
+}
+
 // RandomSampler::Random1D (src/RandomSampler.cuh:681-697), with the
 // dimension's wrap of HaltonSampler::Random1D (:430-439) and
 // SobolSampler::Random1D (:533-545).
 __device__ __forceinline__ float sample1d(PathSampler& s, const DeviceScene& S) {
   const uint32_t type = S.sampler_type;
   const float r = sampler_value(s, type, type == kSamplerHalton ? S.halton_perm : S.sobol_matrices);
-  ++s.dim;
-  if (type == kSamplerHalton) {
-    if (s.dim >= (uint32_t)kHaltonDims) s.dim = 2;
-  } else if (type == kSamplerSobol) {
-    if (s.dim >= 4096u) s.dim = 1;  // the reference wraps here (and prints a warning)
-  }
+  s.dim = next_dim(s.dim, type);
   return r;
 }
 
-// Two / three draws bound to argument positions in the reference's order.
-__device__ __forceinline__ void sample2d(PathSampler& s, const DeviceScene& S, float* a0, float* a1) {
-  if (kDrawLeftToRight) {
-    *a0 = sample1d(s, S);
-    *a1 = sample1d(s, S);
-  } else {
-    *a1 = sample1d(s, S);
-    *a0 = sample1d(s, S);
+// Samples of `n` (2 or 3) consecutive dimensions. The digits of a Halton index
+// come one after the other, each a division and a table read; three bases
+// side by side wait for them together (shading of Cornell 256x256 16 spp 1.27
+// -> 1.19 ms, of the instanced 1080p 64-spp frame 40.9 -> 39.4 ms, of the
+// volumetric 1280x720 16-spp one 167 -> 161 ms).
+static __device__ __noinline__ float3 sampler_values(PathSampler s, uint32_t sampler_type,
+                                                     const uint32_t* __restrict__ table, int n) {
+  float r[3] = {0.0f, 0.0f, 0.0f};
+  if (sampler_type == kSamplerHalton && s.index <= 0xFFFFFFFFull) {
+    uint32_t dim = s.dim, idx[3], base[3], magic[3], shift[3];
+    const uint32_t* perm[3];
+    float inv[3], scale[3];
+    uint64_t sum[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const HaltonDim D = g_halton.dim[dim];
+      idx[k] = k < n ? (uint32_t)s.index : 0u;
+      base[k] = D.base;
+      magic[k] = D.magic;
+      shift[k] = 31u - (uint32_t)__clz((int)(D.base - 1u));
+      perm[k] = table + D.offset;
+      inv[k] = D.inv_base;
+      scale[k] = 1.0f;
+      sum[k] = 0;
+      dim = next_dim(dim, kSamplerHalton);
+    }
+#pragma unroll 2
+    while (idx[0] | idx[1] | idx[2]) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const uint32_t next = divide_by_base(idx[k], magic[k], shift[k]);
+        const uint32_t digit = __ldg(perm[k] + (idx[k] - next * base[k]));
+        if (idx[k]) {
+          sum[k] = sum[k] * base[k] + digit;
+          scale[k] *= inv[k];
+        }
+        idx[k] = next;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float postfix_zero = (float)__ldg(perm[k]) * scale[k] * inv[k] / (1.0f - inv[k]);
+      r[k] = gmax(0.000001f, gmin(__ull2float_rn(sum[k]) * scale[k] + postfix_zero, 0.999999f));
+    }
+    return make_float3(r[0], r[1], r[2]);
   }
+#pragma unroll 1
+  for (int k = 0; k < n; ++k) {
+    const float v = sampler_value(s, sampler_type, table);
+    if (k == 0) r[0] = v;
+    else if (k == 1) r[1] = v;
+    else r[2] = v;
+    s.dim = next_dim(s.dim, sampler_type);
+  }
+  return make_float3(r[0], r[1], r[2]);
 }
-__device__ __forceinline__ void sample3d(PathSampler& s, const DeviceScene& S, float* a0, float* a1, float* a2) {
-  if (kDrawLeftToRight) {
-    *a0 = sample1d(s, S);
-    *a1 = sample1d(s, S);
-    *a2 = sample1d(s, S);
-  } else {
-    *a2 = sample1d(s, S);
-    *a1 = sample1d(s, S);
-    *a0 = sample1d(s, S);
-  }
+
+// Two or three draws, the first bound to the first argument (the reference's
+// argument order as the device front end evaluates it).
+__device__ __forceinline__ float3 sample_next(PathSampler& s, const DeviceScene& S, int n) {
+  static_assert(kDrawLeftToRight, "the first draw is the first argument");
+  const uint32_t type = S.sampler_type;
+  const float3 v = sampler_values(s, type, type == kSamplerHalton ? S.halton_perm : S.sobol_matrices, n);
+  for (int k = 0; k < n; ++k) s.dim = next_dim(s.dim, type);
+  return v;
+}
+__device__ __forceinline__ void sample2d(PathSampler& s, const DeviceScene& S, float* a0, float* a1) {
+  const float3 v = sample_next(s, S, 2);
+  *a0 = v.x;
+  *a1 = v.y;
 }
 
 // RadicalInversion2 / RadicalInversion3 (un-permuted), src/RandomSampler.cuh:481-507.

@@ -431,9 +431,20 @@ __global__ void k_debug_halton(uint32_t slot, int n, const int* px, const int* p
   offset[2 * i] = gmin(gmax(ox, 0.000001f), 0.999999f);
   offset[2 * i + 1] = gmin(gmax(oy, 0.000001f), 0.999999f);
   PathSampler hs{idx, 2u, 0u};
-  for (int d = 0; d < n_dims; ++d) {
-    dims[(size_t)i * n_dims + d] = sampler_value(hs, kSamplerHalton, S.halton_perm);
-    if (++hs.dim >= (uint32_t)kHaltonDims) hs.dim = 2;
+  // both ways the kernels draw: three or two dimensions at a time, and one
+  for (int d = 0; d < n_dims;) {
+    float* out = dims + (size_t)i * n_dims + d;
+    const int n = gmin(n_dims - d, 3 - (d / 6) % 2);
+    if (n == 1) {
+      out[0] = sampler_value(hs, kSamplerHalton, S.halton_perm);
+    } else {
+      const float3 v = sampler_values(hs, kSamplerHalton, S.halton_perm, n);
+      out[0] = v.x;
+      out[1] = v.y;
+      if (n == 3) out[2] = v.z;
+    }
+    for (int k = 0; k < n; ++k) hs.dim = next_dim(hs.dim, kSamplerHalton);
+    d += n;
   }
 }
 

@@ -561,9 +561,8 @@ struct ChosenLight {
   LightTri tri;     // shape lights
 };
 template <uint32_t kF>
-__device__ __forceinline__ void choose_light(const DeviceScene& S, bool distant, PathSampler& hs, ChosenLight& L) {
+__device__ __forceinline__ void choose_light(const DeviceScene& S, bool distant, float u, ChosenLight& L) {
   L.distant = distant;
-  const float u = sample1d(hs, S);
   if (distant) {
     L.select_pdf = 1.0f / float(S.distant_light_count);
     L.index = gmax(gmin((int)(u * S.distant_light_count), (int)S.distant_light_count - 1), 0);
@@ -997,7 +996,6 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
       }
       if (on) {
         if (pass == 0) {
-          choose_light<kF>(S, distant, hs, L);
           direct = vec3(0.0f);
         } else if (kPhased) {
           reload_light<kF>(S, distant, L);
@@ -1009,11 +1007,11 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
         float spdf = 0.0f, maxd = kTMax;  // spdf: of the BSDF or the phase functions
         bool ok = on, tb = false;
         if (on) {
-          float u0, u1, u2 = 0.0f;
-          sample2d(hs, S, &u0, &u1);
-          if (surface && pass == 1) u2 = sample1d(hs, S);
+          // pass 0: the light's choice and a point on it; pass 1: a direction
+          const float3 u = sample_next(hs, S, pass == 0 || surface ? 3 : 2);
           if (pass == 0) {
-            ok = sample_chosen_light<kF>(S, L, sp.p, u0, u1, q);
+            choose_light<kF>(S, distant, u.x, L);
+            ok = sample_chosen_light<kF>(S, L, sp.p, u.y, u.z, q);
             if (ok) {
               if (!kVol || surface) {
                 lwi = B.to_local(q.dir);
@@ -1025,11 +1023,11 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
             }
           } else {
             if (!kVol || surface) {
-              ok = bsdf_sample(B, wo, &f, &lwi, &spdf, u0, u1, u2);
+              ok = bsdf_sample(B, wo, &f, &lwi, &spdf, u.x, u.y, u.z);
               if (ok) q.dir = B.to_world(lwi);
             } else {
               float pw = 0.0f;
-              ok = sample_mixed_phases(vw, gs, n_media, u0, u1, -rd, &pw, &q.dir, &spdf);
+              ok = sample_mixed_phases(vw, gs, n_media, u.x, u.y, -rd, &pw, &q.dir, &spdf);
               f = vec3(pw);
             }
             if (ok) {
@@ -1114,17 +1112,15 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
 
     // The continuation: a direction from the BSDF or the phase functions.
     if (last && (surface || (kVol && volume))) {
-      float u0, u1, u2 = 0.0f;
-      sample2d(hs, S, &u0, &u1);
+      const float3 u = sample_next(hs, S, surface ? 3 : 2);
       vec3 w(0.0f), wi(0.0f);
       float pdf = 0.0f;
       bool valid;
       if (!kVol || surface) {
-        u2 = sample1d(hs, S);
-        valid = bsdf_sample(B, wo, &w, &wi, &pdf, u0, u1, u2);
+        valid = bsdf_sample(B, wo, &w, &wi, &pdf, u.x, u.y, u.z);
       } else {
         float pw = 0.0f;
-        valid = sample_mixed_phases(vw, gs, n_media, u0, u1, -rd, &pw, &wi, &pdf);
+        valid = sample_mixed_phases(vw, gs, n_media, u.x, u.y, -rd, &pw, &wi, &pdf);
         w = vec3(pw);
       }
       if constexpr (kAdj) {
