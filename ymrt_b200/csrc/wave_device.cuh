@@ -135,11 +135,18 @@ __device__ __forceinline__ void file_bucket(WaveCounters* counters, uint32_t buc
 // Launched with kTraceBlock threads by default, or any block size up to
 // kMaxTraceBlock (YMRT_OPT_TRACE_BLOCK, tuned by ymrt_b200.autotune); the
 // traversal stacks are in dynamic shared memory (traversal_shared_bytes).
-// The launch bounds give 128 registers, four resident 128-thread blocks per
-// SM: on the 1080p instanced frame 3.3% faster than five (102 registers,
-// spills in the traversal loop) and 15% faster than three.
+// Registers a thread: 96, five resident 128-thread blocks per SM (instanced
+// 1080p 64 spp, closest hits 97.8 ms at 128 registers and 86.7 at 96, 107 at
+// 80; Cornell 256x256 16 spp 1.07 and 0.97; media with fBm 47.7 and 46.4). The
+// media instantiation with every texture node spills at 96: 128 (smoke grid
+// 33.2 and 34.2 ms).
+template <bool kVol, uint32_t kF>
+constexpr uint32_t extend_registers() {
+  return kVol && (kF & (kFeatGrids | kFeatTextures)) ? 128 : 96;
+}
+
 template <bool kVol, uint32_t kF, bool kAdj = false>
-__global__ void __launch_bounds__(kMaxTraceBlock, 4 * kTraceBlock / kMaxTraceBlock) k_extend(PathPool P, const WaveControl* __restrict__ ctl, HitPool H,
+__global__ void __maxnreg__((extend_registers<kVol, kF>())) k_extend(PathPool P, const WaveControl* __restrict__ ctl, HitPool H,
                                                            const JobDesc* __restrict__ jobs, WaveCounters* counters,
                                                            float* grid_grads = nullptr, uint32_t grid_tex = kEmpty,
                                                            const uint32_t* __restrict__ ray_order = nullptr) {
