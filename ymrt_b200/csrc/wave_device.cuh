@@ -617,8 +617,9 @@ __device__ __forceinline__ void eval_chosen_light(const DeviceScene& S, const Ch
 // and each material vertex adds its terms of dLoss/dParam (see AdjCtx) to
 // `grads` (per-block sums in shared memory, then one atomic per touched slot).
 //
-// The block works stage by stage: fetch the vertex, build its BSDF, and for
-// each of the (up to four) shadow rays set it up, then trace it, then the
+// The block works stage by stage: fetch the vertex, build its BSDF (mapped
+// frame, textured parameters, lobes), and for each of the (up to four) shadow
+// rays set it up, test its occlusion, follow its transmittance, then the
 // continuation, with a barrier between the stages. The kernel is 150-470 KB of
 // code, more than an SM's instruction caches hold, and warps left to run on
 // their own spread over all of it: they waited for instructions 21-32 of 28-40
@@ -633,7 +634,11 @@ __device__ __forceinline__ void eval_chosen_light(const DeviceScene& S, const Ch
 // shading 48.4 ms without barriers, 41.3 at 128, 40.5 at 256, 42.6 at 512;
 // Cornell 256x256 16 spp 1.28, 1.31, 1.37, 1.45 ms). Surface adjoint 256
 // threads (41.1 ms for 4 views 512x512 16 spp; 61.7 without barriers, 46.9 at
-// 128, 43.5 at 512).
+// 128, 43.5 at 512). Finer stages where they are the long ones: occlusion and
+// transmittance apart (shading of the fog gradients' forward pass 12.1 ->
+// 11.3 ms, of solid textures 44.8 -> 43.1), mapped frame and parameters apart
+// (44.8 -> 42.1, image textures 11.65 -> 11.3); one between a light's sampling
+// and its BSDF value gained nothing.
 template <bool kVol, bool kDefer, bool kAdj, uint32_t kF>
 constexpr uint32_t shade_threads() {
   if (kVol || (kF & kFeatTextures)) return 512;
@@ -914,23 +919,26 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
         if (surface) load_adjoint(X, t_idx, adj_ctx);
       }
     }
-    if (first && surface) {
-      const DefaultMtl& md = S.materials[material].default_mtl;
-      const DefaultMtl* mp = &md;
-      DefaultMtl mt;
-      bool plain = true;
-      if constexpr ((kF & kFeatTextures) != 0) {
-        if (material_textured(md)) {
+    bool plain = true;
+    DefaultMtl mt;
+    if constexpr ((kF & kFeatTextures) != 0) {
+      if (first) {
+        const TexCoord tc{sp.u, sp.v, sp.p_obj};
+        const bool textured = surface && material_textured(S.materials[material].default_mtl);
+        if (textured) {
           // textured parameters, normal or bump mapping: read at the hit
-          mt = md;
-          const TexCoord tc{sp.u, sp.v, sp.p_obj};
+          mt = S.materials[material].default_mtl;
           init_shading_frame_mapped(B, mt, hit_back, rd, sp, S.i_transforms[S.instances[inst_idx].transform_idx], S, tc,
                                     errors);
-          resolve_material_textures(mt, S.textures, tc, errors);
-          mp = &mt;
           plain = false;
         }
+        __syncthreads();
+        if (textured) resolve_material_textures(mt, S.textures, tc, errors);
+        __syncthreads();
       }
+    }
+    if (first && surface) {
+      const DefaultMtl* mp = plain ? &S.materials[material].default_mtl : &mt;
       if (plain) init_shading_frame(B, hit_back, rd, sp.ng, sp.ns, sp.dpdu, sp.dpdv);
       init_layered_lobes(B, *mp, rd, hit_back, ray_ior(rt), ex_ior(rt, inst_idx));
       if constexpr (kAdj) {
@@ -1095,17 +1103,17 @@ __global__ void __launch_bounds__(shade_threads<kVol, kDefer, kAdj, kF>(), shade
           if (ok) X.queue[at] = t_idx;
         } else {
           __syncthreads();
+          const vec3 dir = normalize(q.dir);
+          if (ok) ok = !trace_occluded_impl<kSpheres>(slot, st, so, dir, maxd, &tests, &nodes);
+          if (kVol) __syncthreads();
           if (ok) {
-            const vec3 dir = normalize(q.dir);
-            if (!trace_occluded_impl<kSpheres>(slot, st, so, dir, maxd, &tests, &nodes)) {
-              vec3 tr(1.0f);
-              if (kVol && (volume || rs.enable_volume_scattering)) {
-                RayTransfer srt = rt;
-                if (tb) boundary_transition(S, srt, nb, n_nb, errors);
-                tr = trace_tr<kF>(slot, st, so, dir, maxd, inst_idx, tri, srt, hs, errors, &tests, &nodes);
-              }
-              direct += mis * tr * fc * Lc;
+            vec3 tr(1.0f);
+            if (kVol && (volume || rs.enable_volume_scattering)) {
+              RayTransfer srt = rt;
+              if (tb) boundary_transition(S, srt, nb, n_nb, errors);
+              tr = trace_tr<kF>(slot, st, so, dir, maxd, inst_idx, tri, srt, hs, errors, &tests, &nodes);
             }
+            direct += mis * tr * fc * Lc;
           }
           __syncthreads();
         }
