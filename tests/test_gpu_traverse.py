@@ -47,7 +47,17 @@ def brute_force(tri, o, d):
 @pytest.mark.parametrize("scene", ["cornell", "volumetric", "glossy"])
 @pytest.mark.parametrize("n", [1, 31, 33, 129, 1500])
 def test_against_brute_force(ctx, scene, n, halton_perm, scene_dir):
-    host = Y.HostScene(scenes.scene_path(scene, 3, scene_dir), 64, 64)
+    check(ctx, scene, n, halton_perm, scene_dir, 3)
+
+
+@pytest.mark.parametrize("leaf", [1, 2, 4])
+def test_leaf_sizes(ctx, leaf, halton_perm, scene_dir):
+    """Leaves of one to four triangles, and of as many instances in the top level."""
+    check(ctx, "volumetric", 1000, halton_perm, scene_dir, leaf)
+
+
+def check(ctx, scene, n, halton_perm, scene_dir, leaf):
+    host = Y.HostScene(scenes.scene_path(scene, 3, scene_dir), 64, 64, max_leaf_triangles=leaf)
     sc = Y.Scene(ctx, host, halton_perm)
     tri, boundary, owner, index = world_triangles(host)
     rng = np.random.default_rng(n)

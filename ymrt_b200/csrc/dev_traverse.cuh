@@ -35,10 +35,11 @@ constexpr int kMaxTraceBlock = 256;  // largest block k_extend and k_connect are
 
 // Stack entries carry the entry distance of the box that produced them, so a
 // pop can drop entries that lie beyond the current closest hit. An entry is a
-// node index, or (kInstanceEntry set) a group of one to three instances of a
-// top-level leaf: their count in bits 29-30 and the first one's leaf slot.
+// node index, or (kInstanceEntry set) a group of the one to seven instances of
+// a top-level leaf (a node's meta byte has three bits for them): their count
+// in bits 28-30 and the first one's leaf slot.
 constexpr uint32_t kInstanceEntry = 0x80000000u;
-constexpr uint32_t kEntryCountShift = 29, kEntrySlotMask = (1u << kEntryCountShift) - 1u;
+constexpr uint32_t kEntryCountShift = 28, kEntrySlotMask = (1u << kEntryCountShift) - 1u;
 
 struct TraversalStack {
   uint2* sh;  // shared-memory column of this thread: entry, entry distance (stride: the block's threads)
@@ -479,7 +480,7 @@ struct ClosestWalk {
     if (etn > widened_tmax(t_ray)) return kWalkGoing;
     if (e & kInstanceEntry) {
       // the group's last instance now, the others after it
-      const uint32_t count = (e >> kEntryCountShift) & 3u, at = e & kEntrySlotMask;
+      const uint32_t count = (e >> kEntryCountShift) & 7u, at = e & kEntrySlotMask;
       if (count > 1) st.push(e - (1u << kEntryCountShift), etn);
       const EnteredInstance in = enter_instance(S.inst_slots, at + count - 1, wo, wd);
       if (kVolumeOnly && !(in.flags & kSlotBoundary)) return kWalkGoing;
@@ -662,7 +663,7 @@ __device__ __forceinline__ int occluded_step(OccWalk& w, Stack& st, uint32_t* tr
     e = st.pop();
   }
   if (e & kInstanceEntry) {
-    const uint32_t count = (e >> kEntryCountShift) & 3u, at = e & kEntrySlotMask;
+    const uint32_t count = (e >> kEntryCountShift) & 7u, at = e & kEntrySlotMask;
     if (count > 1) st.push(e - (1u << kEntryCountShift));
     const EnteredInstance in = enter_instance(S.inst_slots, at + count - 1, w.wo, w.wd);
     if (in.flags & kSlotBoundary) return kWalkGoing;
