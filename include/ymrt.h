@@ -131,7 +131,8 @@ int ymrt_set_profiling(ymrt_context* ctx, int enable);
 #define YMRT_OPT_TRACE_BLOCK 4
 /*   YMRT_OPT_SORT_RAYS     (default 1) trace each wave's continuing rays
  *                          grouped by origin cell and direction instead of
- *                          in the order shading left them (same hits) */
+ *                          in the order shading left them (same hits), in
+ *                          waves of at least 131,072 of them */
 #define YMRT_OPT_SORT_RAYS 6
 int ymrt_set_option(ymrt_context* ctx, int option, int value);
 int ymrt_get_option(const ymrt_context* ctx, int option, int* value);

@@ -5,10 +5,12 @@
 //               still alive (Ray_generation_path_tracing, src/Shading.cu:1634);
 //   extend   -> closest hit for every live path; misses are accumulated and
 //               retired (Ray_trace_path_tracing, src/Shading.cu:1765);
-//   shade    -> hit reconstruction, next-event estimation with both shadow
-//               rays traced in place, BSDF continuation; surviving paths are
-//               compacted into the other pool with one atomic per warp
-//               (Ray_shading_path_tracing, src/Shading.cu:1953).
+//   shade    -> hit reconstruction, next-event estimation (surface shadow rays
+//               queued for connect, with media traced in place), BSDF or
+//               phase-function continuation; surviving paths are compacted
+//               into the other pool with one atomic per warp
+//               (Ray_shading_path_tracing, src/Shading.cu:1953);
+//   connect  -> the queued shadow rays.
 // Path state is structure-of-arrays (float4 / uint2 per field) so every
 // field of a wave is read and written with coalesced 16-byte accesses.
 //

@@ -612,7 +612,7 @@ __device__ __forceinline__ void eval_chosen_light(const DeviceScene& S, const Ch
 // for k_connect instead of traced here, which keeps traversal out of this
 // kernel.
 //
-// kAdj (surfaces, inline shadow rays): the path-replay adjoint pass. Paths
+// kAdj: the path-replay adjoint pass, in phases (launch_shade_phases). Paths
 // are shaded exactly as in the forward pass, nothing is added to the image,
 // and each material vertex adds its terms of dLoss/dParam (see AdjCtx) to
 // `grads` (per-block sums in shared memory, then one atomic per touched slot).
