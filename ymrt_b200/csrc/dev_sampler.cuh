@@ -96,9 +96,37 @@ __device__ __forceinline__ uint64_t halton_index(const DeviceScene& S, int px, i
   return off + (uint64_t)ith_sample * (uint64_t)S.halton_increment;
 }
 
+// The digits of an index above 32 bits, one 64-bit division each, until 32
+// bits hold the rest (a progressive 1080p 64-spp render passes 2^32 in its
+// 15th frame, and then has one to four such digits). Below 2^44 the quotient
+// is a double product: inv is within 2^-47 of 1 / base, so the product is
+// within one of the quotient and the remainder corrects it (instanced 1080p 64
+// spp, frame 40: 178.7 -> 174.7 ms).
+__device__ __forceinline__ uint32_t reduce_index(uint64_t index, uint32_t base, float inv_base,
+                                                 const uint32_t* __restrict__ perm, uint64_t* sum, float* scale) {
+  if (index >> 32) {
+    const double b = (double)base, inv0 = (double)inv_base;
+    const double inv = __fma_rn(inv0, __fma_rn(-b, inv0, 1.0), inv0);
+#pragma unroll 1
+    do {
+      uint64_t next;
+      if (index < (1ull << 44)) {
+        next = (uint64_t)((double)index * inv);
+        const int64_t rem = (int64_t)(index - next * base);
+        if (rem < 0) --next;
+        else if (rem >= (int64_t)base) ++next;
+      } else {
+        next = index / base;
+      }
+      *sum = *sum * base + __ldg(perm + (uint32_t)(index - next * base));
+      *scale *= inv_base;
+      index = next;
+    } while (index >> 32);
+  }
+  return (uint32_t)index;
+}
+
 // RadicalInversion with a digit permutation, src/RandomSampler.cuh:462-480.
-// Indices below 2^32 (every sample of a 4K frame at 64 spp) take the 32-bit
-// division path; the digits, and therefore the result, are identical.
 __device__ __forceinline__ float radical_inverse_perm(uint64_t index, const HaltonDim& D,
                                                       const uint32_t* __restrict__ table) {
   const uint32_t base = D.base;
@@ -106,15 +134,7 @@ __device__ __forceinline__ float radical_inverse_perm(uint64_t index, const Halt
   const uint32_t* __restrict__ perm = table + D.offset;
   uint64_t radical_sum = 0;
   float base_multiply = 1.0f;
-#pragma unroll 1
-  while (index > 0xFFFFFFFFull) {
-    const uint64_t next = index / base;
-    const uint64_t digit = index - next * base;
-    radical_sum = radical_sum * base + __ldg(perm + digit);
-    base_multiply *= inv_base;
-    index = next;
-  }
-  uint32_t idx = (uint32_t)index;
+  uint32_t idx = reduce_index(index, base, inv_base, perm, &radical_sum, &base_multiply);
   const uint32_t shift = 31u - (uint32_t)__clz((int)(base - 1u));  // ceil(log2 base) - 1
   while (idx) {
     const uint32_t next = divide_by_base(idx, D.magic, shift);
@@ -236,7 +256,7 @@ __device__ __forceinline__ float sample1d(PathSampler& s, const DeviceScene& S) 
 static __device__ __noinline__ float3 sampler_values(PathSampler s, uint32_t sampler_type,
                                                      const uint32_t* __restrict__ table, int n) {
   float r[3] = {0.0f, 0.0f, 0.0f};
-  if (sampler_type == kSamplerHalton && s.index <= 0xFFFFFFFFull) {
+  if (sampler_type == kSamplerHalton) {
     uint32_t dim = s.dim, idx[3], base[3], magic[3], shift[3];
     const uint32_t* perm[3];
     float inv[3], scale[3];
@@ -244,7 +264,6 @@ static __device__ __noinline__ float3 sampler_values(PathSampler s, uint32_t sam
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const HaltonDim D = g_halton.dim[dim];
-      idx[k] = k < n ? (uint32_t)s.index : 0u;
       base[k] = D.base;
       magic[k] = D.magic;
       shift[k] = 31u - (uint32_t)__clz((int)(D.base - 1u));
@@ -252,6 +271,7 @@ static __device__ __noinline__ float3 sampler_values(PathSampler s, uint32_t sam
       inv[k] = D.inv_base;
       scale[k] = 1.0f;
       sum[k] = 0;
+      idx[k] = k < n ? reduce_index(s.index, D.base, D.inv_base, perm[k], &sum[k], &scale[k]) : 0u;
       dim = next_dim(dim, kSamplerHalton);
     }
 #pragma unroll 2
@@ -304,23 +324,10 @@ __device__ __forceinline__ void sample2d(PathSampler& s, const DeviceScene& S, f
 // Camera rays draw these two and the pixel's index only, in 64-bit loops of
 // divisions that took half of k_generate (7.8 -> 4.2 ms of the instanced 1080p
 // 64-spp frame with the 32-bit forms below).
-// Indices below 2^32 (as in radical_inverse_perm) need no loop in base 2: the
-// n digits in reverse, rounded to a float and scaled by 2^-n, are the whole
-// word's reversal rounded and scaled by 2^-32.
+// Base 2 needs no loop: the n digits in reverse, rounded to a float and scaled
+// by 2^-n, are the whole word's reversal rounded and scaled by 2^-64.
 __device__ __forceinline__ float radical_inverse_2(uint64_t index) {
-  if (index <= 0xFFFFFFFFull)
-    return gmax(0.000001f, gmin(__uint2float_rn(__brev((uint32_t)index)) * (1.0f / 4294967296.0f), 0.999999f));
-  const float inv_base = 1.0f / float(2u);
-  uint64_t radical_sum = 0;
-  float base_multiply = 1.0f;
-  while (index) {
-    const uint64_t next = index / 2u;
-    const uint64_t digit = index - next * 2u;
-    radical_sum = radical_sum * 2u + digit;
-    base_multiply *= inv_base;
-    index = next;
-  }
-  return gmax(0.000001f, gmin(__ull2float_rn(radical_sum) * base_multiply, 0.999999f));
+  return gmax(0.000001f, gmin(__ull2float_rn(__brevll(index)) * 5.42101086242752217e-20f, 0.999999f));
 }
 __device__ __forceinline__ float radical_inverse_3(uint64_t index) {
   const float inv_base = 1.0f / float(3u);
