@@ -1188,10 +1188,19 @@ uint32_t batch_features(const DeviceScene* scenes, size_t n) {
   return f;
 }
 
-// Bits that tell n scenes apart (n <= kMaxSceneSlots: at most 6).
-uint32_t scene_bits(size_t n) {
+// Bits of a scene's slot that the grouping of continuing rays leads with
+// (each taken from the resolution of its cells). Jobs enter the waves in path
+// order and their slots are consecutive, so it is enough to tell the scenes
+// apart that share a wave: those whose paths fill the pool, twice over for
+// the long paths of earlier ones. 64 renders of 15 M paths each need 2 bits
+// (2496 ms with all 6, 2290 with 2), 48 previews of 0.15 M 5.
+uint32_t scene_bits(size_t scenes, const std::vector<JobDesc>& jobs, uint32_t capacity) {
+  unsigned long long paths = 0;
+  for (const JobDesc& j : jobs) paths += j.path_count;
+  const unsigned long long each = std::max<unsigned long long>(paths / std::max<size_t>(scenes, 1), 1);
+  const unsigned long long together = std::min<unsigned long long>(scenes, 2ull * capacity / each + 2);
   uint32_t bits = 0;
-  while ((size_t(1) << bits) < n) ++bits;
+  while ((1ull << bits) < together) ++bits;
   return bits;
 }
 
@@ -1339,7 +1348,7 @@ int ymrt_render_batch(ymrt_context* ctx, const ymrt_job* jobs_in, int n_jobs, ym
     WaveOptions opt;
     if ((rc = batch_options(ctx, jobs, &opt)) != YMRT_OK) return rc;
     opt.features = batch_features(slots.data(), slots.size());
-    opt.scene_bits = scene_bits(slots.size());
+    opt.scene_bits = scene_bits(slots.size(), jobs, M.capacity);
     SlotLease lease(ctx, (uint32_t)slots.size());
     if (!lease.ok()) return ctx->fail(YMRT_ERR_INVALID, "no constant-memory scene slots for this device");
     for (JobDesc& j : jobs) j.scene_slot = lease.slot(j.scene_slot);
@@ -1417,7 +1426,7 @@ int ymrt_render_backward_ex(ymrt_context* ctx, const ymrt_job* jobs_in, int n_jo
   opt.trace_block = ctx->trace_block;
   opt.sort_rays = ctx->sort_rays;
   opt.features = batch_features(slots.data(), slots.size());
-  opt.scene_bits = scene_bits(slots.size());
+  opt.scene_bits = scene_bits(slots.size(), jobs, M.capacity);
   opt.grads = materials ? tg->material_grads_device : nullptr;
   opt.grad_materials = materials ? tg->n_materials : 0;
   opt.grid_grads = grid ? tg->grid_grads_device : nullptr;

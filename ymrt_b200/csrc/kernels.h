@@ -241,7 +241,7 @@ struct WaveOptions {
   bool volumes = false;        // volume scattering kernels
   bool sort_hits = true;       // shade hits listed by shading bucket
   bool sort_rays = false;      // trace continuing rays grouped by origin cell and direction
-  uint32_t scene_bits = 0;     // ceil(log2) of the batch's distinct scenes: the grouping keeps them apart
+  uint32_t scene_bits = 0;     // bits of the scene's slot that lead the grouping's key (0: one scene)
   bool defer_shadows = false;  // queue surface shadow rays for k_connect (ignored with volumes)
   uint32_t features = kFeatAll;  // scene features of the batch (kFeatSpheres | kFeatGrids | kFeatTextures)
   VertexQueue vertices{};        // adjoint: vertices between the phases of k_shade
