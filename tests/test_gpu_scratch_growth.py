@@ -1,0 +1,50 @@
+"""Scratch memory that grows on demand, when growing fails (host-side
+injection, ymrt_debug_fail_allocations): the old block is gone then, so a
+later call that the old one would have sufficed for has to allocate anew. That
+is checked on the host first (with allocations failing it returns
+YMRT_ERR_OOM instead of using freed memory), and only then on the device."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import ymrt_b200 as Y
+
+pytestmark = pytest.mark.gpu
+
+OOM = -6  # YMRT_ERR_OOM
+
+
+class failing_allocations:
+    def __enter__(self):
+        Y.library().ymrt_debug_fail_allocations(1000)
+
+    def __exit__(self, *exc):
+        Y.library().ymrt_debug_fail_allocations(0)
+
+
+def backward(ctx, scene, spp):
+    import torch
+    w, h = scene.width, scene.height
+    render = [scene, Y.default_setting(spp=spp, ray_depth=8), 1, torch.zeros((h, w, 4), device="cuda")]
+    record = torch.zeros((Y.path_count(render), 4), device="cuda")
+    grads = torch.zeros((scene.material_params().shape[0], 4), device="cuda")
+    torch.cuda.synchronize()
+    Y.render_batch(ctx, [render], [record])
+    dloss = torch.ones_like(render[3])
+    torch.cuda.synchronize()
+    return lambda: (Y.render_backward(ctx, [render], [record], [dloss], grads), grads.cpu().numpy().copy())[1]
+
+
+def test_backward_after_a_failed_larger_one(cornell_path, halton_perm):
+    with Y.Context(0) as c:
+        scene = Y.Scene(c, Y.HostScene(cornell_path, 64, 48), halton_perm)
+        small, large = backward(c, scene, 1), backward(c, scene, 32)
+        want = small()
+        for step in (large, small):  # the larger grows the vertices; the smaller then has none left
+            with failing_allocations(), pytest.raises(Y.YmrtError) as e:
+                step()
+            assert e.value.code == OOM
+        # dLoss/dImage = 1: positive terms, at most 64 * 48 pixels x 8 vertices of them, 2.5e4 * 2^-24 = 1.5e-3
+        np.testing.assert_allclose(small()[:, :3], want[:, :3], rtol=1.5e-3, atol=1e-6)
+        assert large()[:, :3].max() > 0

@@ -226,6 +226,7 @@ struct ymrt_context {
     while (n < pool_capacity && n < paths) n *= 2;
     n = std::min<size_t>(n, pool_capacity);
     if (vertices.capacity >= n) return YMRT_OK;
+    vertices = VertexQueue{};  // growing frees the old block first: no view of it may outlive a failure
     const size_t words = kVertexStateWords + kVertexLobeWords + kVertexAdjointWords + kVertexPassWords + 3;
     cudaError_t e = vertex_buf.ensure(n * (words * sizeof(uint4) + 4 * sizeof(uint32_t)));
     if (e != cudaSuccess) return cuda_fail(e, "allocating shading vertices");
