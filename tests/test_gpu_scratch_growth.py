@@ -48,3 +48,20 @@ def test_backward_after_a_failed_larger_one(cornell_path, halton_perm):
         # dLoss/dImage = 1: positive terms, at most 64 * 48 pixels x 8 vertices of them, 2.5e4 * 2^-24 = 1.5e-3
         np.testing.assert_allclose(small()[:, :3], want[:, :3], rtol=1.5e-3, atol=1e-6)
         assert large()[:, :3].max() > 0
+
+
+def test_queues_after_a_failed_larger_capacity(cornell_path, halton_perm):
+    """A program that goes back to its old queue capacity when a larger one does not fit."""
+    with Y.Context(0, queue_capacity=1 << 14) as c:
+        scene = Y.Scene(c, Y.HostScene(cornell_path, 64, 48), halton_perm)
+        setting = Y.default_setting(spp=4, ray_depth=8)
+        want, _ = scene.render(setting, 1)
+        for capacity in (1 << 16, 1 << 14):
+            Y.library().ymrt_set_queue_capacity(c.h, capacity)
+            with failing_allocations(), pytest.raises(Y.YmrtError) as e:
+                scene.render(setting, 1)
+            assert e.value.code == OOM
+        got, st = scene.render(setting, 1)
+        assert st.device_errors == 0
+        # at most 4 shadow rays at each of 8 vertices, 4 samples: 128 additions in another order, 128 * 2^-24
+        np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-7)

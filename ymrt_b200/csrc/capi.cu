@@ -177,6 +177,11 @@ struct ymrt_context {
 
   int ensure_pools() {
     if (pool_capacity == capacity) return YMRT_OK;
+    // (growing frees the old blocks first: no view of them may outlive a
+    // failure, also when the caller then goes back to the old capacity)
+    pool_capacity = 0;
+    shadow_queue = ShadowQueue{};
+    vertices = VertexQueue{};
     const size_t n = capacity;
     const size_t pool_bytes =
         n * (4 * sizeof(float4) + 2 * sizeof(uint2) + sizeof(uint4) + sizeof(RayTransfer) + sizeof(uint32_t) + 1) + 64;
@@ -214,8 +219,6 @@ struct ymrt_context {
     hits.ray_order = reinterpret_cast<uint32_t*>(h); h += n * sizeof(uint32_t);
     hits.bucket = reinterpret_cast<uint8_t*>(h);
     pool_capacity = capacity;
-    shadow_queue = ShadowQueue{};
-    vertices = VertexQueue{};
     return YMRT_OK;
   }
 
