@@ -108,7 +108,9 @@ int ymrt_create(int device_ordinal, ymrt_context** out);
 void ymrt_destroy(ymrt_context* ctx);
 /* Last error message of the context (or of the library when ctx is NULL). */
 const char* ymrt_last_error(const ymrt_context* ctx);
-/* Largest number of paths in flight (queue slots); 0 keeps the default. */
+/* Largest number of paths in flight (queue slots); 0: the default, 2^21. The
+ * queues take about 600 bytes of device memory a slot, and 210 more for the
+ * deferred shadow rays of surface renders. */
 int ymrt_set_queue_capacity(ymrt_context* ctx, uint32_t paths);
 /* When enabled, every stage launch is bracketed by CUDA events and the
  * per-stage times are reported in ymrt_stats (costs a little host time). */
@@ -338,7 +340,11 @@ unsigned long long ymrt_job_path_count(const ymrt_job* job);
  * path_radiance_device set, with unchanged scenes and settings: every path is
  * re-traced with its own samples. grads_device receives 4 floats per material
  * (n_materials materials, in the scene's material order), overwritten.
- * The indirect clamp is rejected. */
+ * The indirect clamp is rejected.
+ * Device memory: beside the path queues the context keeps 672 bytes for each
+ * path of the call, at most for a queue of them (1.4 GB at the default
+ * capacity of 2^21). Where they do not fit, the pass runs in smaller waves;
+ * YMRT_ERR_OOM when even 1024 paths' do not. */
 int ymrt_render_backward(ymrt_context* ctx, const ymrt_job* jobs, int n_jobs, float* grads_device,
                          uint32_t n_materials, ymrt_stats* stats);
 

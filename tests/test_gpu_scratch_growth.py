@@ -65,3 +65,19 @@ def test_queues_after_a_failed_larger_capacity(cornell_path, halton_perm):
         assert st.device_errors == 0
         # at most 4 shadow rays at each of 8 vertices, 4 samples: 128 additions in another order, 128 * 2^-24
         np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("failures", [1, 3, 7])
+def test_backward_in_smaller_waves_when_memory_is_short(cornell_path, halton_perm, failures):
+    """Room for half the vertices, an eighth, or the least there is: the pass still gives its gradients."""
+    with Y.Context(0) as c:
+        scene = Y.Scene(c, Y.HostScene(cornell_path, 64, 48), halton_perm)
+        step = backward(c, scene, 32)  # 98,304 paths: vertices for 131,072, 65,536, ..., 1024
+        Y.library().ymrt_debug_fail_allocations(failures)
+        try:
+            got = step()
+        finally:
+            Y.library().ymrt_debug_fail_allocations(0)
+        want = step()
+        # each wave adds a block's sums: fewer than 1e6 positive terms, in 1e3 groups of 1e3, 2e3 * 2^-24
+        np.testing.assert_allclose(got[:, :3], want[:, :3], rtol=5e-4, atol=1e-6)

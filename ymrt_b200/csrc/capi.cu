@@ -53,6 +53,7 @@ struct DeviceBuffer {
     if (g_failing_allocations.load() > 0 && g_failing_allocations.fetch_sub(1) > 0) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMalloc(&ptr, n ? n : 16);
     if (e == cudaSuccess) bytes = n;
+    else cudaGetLastError();  // reported here: a later check of launches must not find it
     return e;
   }
   template <typename T>
@@ -222,16 +223,25 @@ struct ymrt_context {
     return YMRT_OK;
   }
 
-  // Vertices between the phases of adjoint shading.
-  // For `paths` paths, at most a pool of them (no wave holds more).
+  // Vertices between the phases of adjoint shading, for `paths` paths, at most
+  // a pool of them (no wave holds more). Where so many do not fit (they take
+  // kVertexBytes, 672, a path), half as many, and so on down
+  // to kMinVertices: the pass then runs in smaller waves (vertices.capacity).
+  static constexpr size_t kMinVertices = 1024;
+  static constexpr size_t kVertexBytes =
+      (kVertexStateWords + kVertexLobeWords + kVertexAdjointWords + kVertexPassWords + 3) * sizeof(uint4) +
+      4 * sizeof(uint32_t);
   int ensure_vertices(unsigned long long paths) {
-    size_t n = 1024;
+    size_t n = kMinVertices;
     while (n < pool_capacity && n < paths) n *= 2;
     n = std::min<size_t>(n, pool_capacity);
     if (vertices.capacity >= n) return YMRT_OK;
     vertices = VertexQueue{};  // growing frees the old block first: no view of it may outlive a failure
-    const size_t words = kVertexStateWords + kVertexLobeWords + kVertexAdjointWords + kVertexPassWords + 3;
-    cudaError_t e = vertex_buf.ensure(n * (words * sizeof(uint4) + 4 * sizeof(uint32_t)));
+    cudaError_t e = vertex_buf.ensure(n * kVertexBytes);
+    while (e == cudaErrorMemoryAllocation && n / 2 >= kMinVertices) {
+      n /= 2;
+      e = vertex_buf.ensure(n * kVertexBytes);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "allocating shading vertices");
     uint4* p = vertex_buf.as<uint4>();
     VertexQueue X{};
@@ -1436,6 +1446,7 @@ int ymrt_render_backward_ex(ymrt_context* ctx, const ymrt_job* jobs_in, int n_jo
   opt.grid_grads = grid ? tg->grid_grads_device : nullptr;
   opt.grid_tex = grid ? tg->grid_texture : kEmpty;
   if ((rc = phase_options(ctx, jobs, &opt)) != YMRT_OK) return rc;
+  M.capacity = std::min(M.capacity, opt.vertices.capacity);  // a wave's vertices have to fit
   SlotLease lease(ctx, (uint32_t)slots.size());
   if (!lease.ok()) return ctx->fail(YMRT_ERR_INVALID, "no constant-memory scene slots for this device");
   for (JobDesc& j : jobs) j.scene_slot = lease.slot(j.scene_slot);
