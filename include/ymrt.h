@@ -507,6 +507,9 @@ int ymrt_debug_bound_record(ymrt_context* ctx, uint32_t* words, size_t n_words, 
  * as out of memory (the call that needs them returns YMRT_ERR_OOM and leaves
  * the context usable); 0 stops it. */
 void ymrt_debug_fail_allocations(int count);
+/* What a context has done, for tests of its bounds: out receives the first n
+ * of: wave loops captured so far, captured loops kept. Returns how many there are. */
+int ymrt_debug_counters(const ymrt_context* ctx, uint64_t* out, size_t n);
 int ymrt_debug_occluded(ymrt_scene* scene, int n, const float* origin, const float* dir, const float* tmax,
                         int* occluded);
 int ymrt_debug_halton(ymrt_scene* scene, int n, const int* px, const int* py, const int* sample, int n_dims,

@@ -159,6 +159,7 @@ def library():
     L.ymrt_debug_occluded.argtypes = [vp, i, vp, vp, vp, vp]
     L.ymrt_debug_halton.argtypes = [vp, i, vp, vp, vp, i, vp, vp, vp]
     L.ymrt_debug_bound_record.argtypes = [vp, vp, sz, i]
+    L.ymrt_debug_counters.argtypes = [vp, vp, sz]
     L.ymrt_debug_fail_allocations.argtypes = [i]
     L.ymrt_debug_fail_allocations.restype = None
     L.ymrt_scene_set_transforms.argtypes = [vp, ctypes.c_uint32, ctypes.c_uint32, vp, vp, vp]
@@ -205,6 +206,14 @@ class Context:
         v = ctypes.c_int()
         _check(library().ymrt_get_option(self.h, OPTIONS[name], ctypes.byref(v)))
         return v.value
+
+    COUNTERS = ("loops_captured", "loops_kept")
+
+    def counters(self) -> dict:
+        """What the context has done (ymrt_debug_counters)."""
+        v = (ctypes.c_uint64 * len(self.COUNTERS))()
+        library().ymrt_debug_counters(self.h, v, len(v))
+        return dict(zip(self.COUNTERS, v))
 
     BOUND_SITES = {1: "shadow-ray boundary crossings", 2: "delta-tracking steps", 3: "ratio-tracking steps",
                    4: "waves of a frame", 5: "editor-view boundaries", 6: "texture-graph walk"}

@@ -79,16 +79,19 @@ struct ymrt_context {
   DeviceBuffer ctl_buf;
   // CUDA graphs of the wave loop (a while-loop node around two waves), kept
   // for the memory, options and grid sizes they were captured with, the last
-  // used first: a program that alternates two or three kinds of call (a forward
-  // and a backward pass, previews and finals) captures each once.
+  // used first: a program that alternates kinds of call (a forward and a
+  // backward pass, previews and finals) captures each once. 16: one kind of
+  // call has at most 12 grid sizes (loop_paths, at the largest queue), so renders
+  // of any sizes in turn, in two kinds at the default queue, capture nothing anew.
   bool graph_loop = true;
   struct WaveGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     std::vector<uintptr_t> key;
   };
-  static constexpr size_t kMaxGraphs = 6;
+  static constexpr size_t kMaxGraphs = 16;
   std::vector<WaveGraph> graphs;
+  uint64_t loops_captured = 0;
   static void destroy_graph(WaveGraph& w) {
     if (w.exec) cudaGraphExecDestroy(w.exec);
     if (w.graph) cudaGraphDestroy(w.graph);
@@ -112,6 +115,7 @@ struct ymrt_context {
       graphs.pop_back();
     }
     graphs.insert(graphs.begin(), std::move(w));
+    ++loops_captured;
   }
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   // the branch of the captured wave loop that traces deferred shadow rays
@@ -1005,6 +1009,19 @@ std::vector<DeviceScene> assign_slots(std::vector<JobDesc>& jobs, const std::vec
   return slots;
 }
 
+// Paths the wave loop's grids are made for: what the batch has, or (no wave
+// holds more) the queue. In powers of four from 1024, so that renders of
+// similar sizes share a captured loop, and a program that renders every size
+// in turn has seven of them at the default queue. A 64x64 1-spp frame, 2^12
+// paths, takes 0.60 ms of device time, 0.71 with grids for the whole queue of
+// 2^21; a capture takes 0.4 ms (twelve sizes from 2^10 to 2^21 in turn: a
+// 2^12 one 0.68 ms, as alone; 1.04 with powers of two and six loops kept).
+uint32_t loop_paths(unsigned long long paths, uint32_t capacity) {
+  unsigned long long n = 1024;
+  while (n < capacity && n < paths) n *= 4;
+  return (uint32_t)std::min<unsigned long long>(n, capacity);
+}
+
 // Renders a batch of jobs (paths numbered job after job). The wave loop is
 // planned on the device (k_plan / k_finish); the host either launches the
 // whole loop as one CUDA graph (a while-loop node around two waves, captured
@@ -1030,6 +1047,7 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
   c.total = total;
   c.capacity = M.capacity;
   c.more = 1;
+  c.scene_bits = opt.scene_bits;
   // a path lives at most kMaxRayDepth scattering vertices plus its boundary
   // crossings: a generous bound on waves, reached only by a fault
   const unsigned long long bound = total / std::max<uint32_t>(M.capacity, 1u) * 80ull + 4096ull;
@@ -1037,12 +1055,7 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
   if ((e = cudaMemcpyAsync(M.ctl, &c, sizeof(c), cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return ctx->cuda_fail(e, "uploading the wave control");
   WaveOptions o = opt;
-  // Grids for the paths there are: a wave never holds more than the batch. A
-  // power of two, so that renders of similar sizes share a captured loop (a
-  // 64x64 1-spp frame, 2^12 paths in a pool of 2^21, 0.71 -> 0.60 ms of device time).
-  o.capacity = 1024;
-  while (o.capacity < M.capacity && o.capacity < total) o.capacity *= 2;
-  o.capacity = std::min(o.capacity, M.capacity);
+  o.capacity = loop_paths(total, M.capacity);
   if ((e = cudaMemsetAsync(M.counters, 0, sizeof(WaveCounters), st)) != cudaSuccess)
     return ctx->cuda_fail(e, "clearing the wave counters");
   if (M.hits.ray_bins && (e = cudaMemsetAsync(M.hits.ray_bins, 0, kRayBins * sizeof(uint32_t), st)) != cudaSuccess)
@@ -1054,7 +1067,7 @@ int run_batch(ymrt_context* ctx, const BatchMemory& M, std::vector<JobDesc>& job
         (uintptr_t)M.pool[0].ray_o, (uintptr_t)M.pool[1].ray_o, (uintptr_t)M.hits.bary_t, (uintptr_t)M.ctl,
         (uintptr_t)M.jobs, (uintptr_t)M.counters, (uintptr_t)jobs.size(), (uintptr_t)o.volumes,
         (uintptr_t)o.sort_hits, (uintptr_t)o.defer_shadows, (uintptr_t)o.shadow_queue.o, M.capacity, o.capacity,
-        (uintptr_t)o.trace_block, (uintptr_t)o.sort_rays, (uintptr_t)o.scene_bits,
+        (uintptr_t)o.trace_block, (uintptr_t)o.sort_rays,
         (uintptr_t)o.features, (uintptr_t)o.grid_grads, (uintptr_t)o.grid_tex,
         (uintptr_t)o.adjoint, (uintptr_t)o.grads, o.grad_materials, (uintptr_t)o.vertices.state, o.vertices.capacity, o.light_kinds};
     ymrt_context::WaveGraph* loop = ctx->find_graph(key);
@@ -2400,6 +2413,13 @@ int ymrt_debug_occluded(ymrt_scene* sc, int n, const float* origin, const float*
   return YMRT_OK;
 }
 
+int ymrt_debug_counters(const ymrt_context* ctx, uint64_t* out, size_t n) {
+  if (!ctx || (!out && n)) return YMRT_ERR_INVALID;
+  const uint64_t v[] = {ctx->loops_captured, ctx->graphs.size()};
+  const size_t have = sizeof(v) / sizeof(v[0]);
+  for (size_t k = 0; k < n; ++k) out[k] = k < have ? v[k] : 0u;
+  return (int)have;
+}
 void ymrt_debug_fail_allocations(int count) { g_failing_allocations.store(count > 0 ? count : 0); }
 
 int ymrt_debug_bound_record(ymrt_context* ctx, uint32_t* words, size_t n_words, int clear) {

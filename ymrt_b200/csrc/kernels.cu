@@ -549,8 +549,8 @@ __device__ __forceinline__ uint32_t ray_group_key(uint32_t slot, uint32_t scene_
 }
 
 __global__ void __launch_bounds__(256) k_ray_hist(PathPool P, const WaveControl* __restrict__ ctl, HitPool H,
-                                                  const JobDesc* __restrict__ jobs, uint32_t scene_bits) {
-  const uint32_t live = grouped_rays(ctl);
+                                                  const JobDesc* __restrict__ jobs) {
+  const uint32_t live = grouped_rays(ctl), scene_bits = ctl->scene_bits;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < live; i += gridDim.x * blockDim.x) {
     const uint2 pf = P.pixel_flags[i];
     const uint32_t key = ray_group_key(jobs[pf.y >> kFlagJobShift].scene_slot, scene_bits, P.ray_o[i], P.ray_d[i]);
@@ -756,7 +756,7 @@ uint32_t launch_wave(const PathPool& A, const PathPool& B, const HitPool& H, Wav
   if (sort_rays) {
     // (the counts are zero: cleared when allocated, at the start of every
     // frame and by each wave's k_ray_scan_blocks)
-    k_ray_hist<<<blocks_256, 256, 0, stream>>>(A, ctl, H, jobs, opt.scene_bits);
+    k_ray_hist<<<blocks_256, 256, 0, stream>>>(A, ctl, H, jobs);
     k_ray_scan_blocks<<<kRayScanBlocks, 1024, 0, stream>>>(ctl, H);
     k_ray_scan_partials<<<1, 1024, 0, stream>>>(ctl, H);
     k_ray_scatter<<<blocks_256, 256, 0, stream>>>(ctl, H);

@@ -202,7 +202,7 @@ struct WaveControl {
   uint32_t waves;                 // waves finished
   uint32_t max_waves;             // bound on waves (then YMRT_DEVERR_ITER)
   uint32_t more;                  // 1 while paths remain
-  uint32_t reserved;
+  uint32_t scene_bits;            // bits of the scene's slot that lead the grouping's key
 };
 
 constexpr int kGradParams = 4;  // differentiated parameters per material: albedo r, g, b, roughness
@@ -241,7 +241,7 @@ struct WaveOptions {
   bool volumes = false;        // volume scattering kernels
   bool sort_hits = true;       // shade hits listed by shading bucket
   bool sort_rays = false;      // trace continuing rays grouped by origin cell and direction
-  uint32_t scene_bits = 0;     // bits of the scene's slot that lead the grouping's key (0: one scene)
+  uint32_t scene_bits = 0;     // WaveControl::scene_bits (0: one scene)
   bool defer_shadows = false;  // queue surface shadow rays for k_connect (ignored with volumes)
   uint32_t features = kFeatAll;  // scene features of the batch (kFeatSpheres | kFeatGrids | kFeatTextures)
   VertexQueue vertices{};        // adjoint: vertices between the phases of k_shade
