@@ -304,6 +304,8 @@ int ymrt_host_scene_set_transforms(ymrt_host_scene* scene, uint32_t first, uint3
 #define YMRT_SCENE_INSTANCE_BUCKETS 6 /* uint8 shading bucket per instance */
 #define YMRT_SCENE_CAMERA_MEDIA 7    /* the camera's RayTransfer, 104 bytes */
 #define YMRT_SCENE_FILE_INDEX 8      /* uint32 file index of each instance */
+#define YMRT_SCENE_TLAS_KINDS 9      /* uint16 per top-level node: children with boundary instances, with others << 8 */
+#define YMRT_SCENE_INSTANCE_SLOTS 10 /* the traversal's record per top-level leaf slot, 64 bytes each */
 long long ymrt_scene_download(const ymrt_scene* scene, int what, void* out, size_t cap_bytes);
 
 /* ---- rendering ---- */

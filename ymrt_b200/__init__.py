@@ -464,7 +464,8 @@ class Scene:
 
     SCENE_PARTS = {"tlas_nodes": (1, np.uint8), "tlas_prims": (2, np.uint32), "instances": (3, np.uint32),
                    "shape_lights": (4, np.uint32), "light_table": (5, np.float32), "instance_buckets": (6, np.uint8),
-                   "camera_media": (7, np.uint32), "file_index": (8, np.uint32)}
+                   "camera_media": (7, np.uint32), "file_index": (8, np.uint32),
+                   "tlas_kinds": (9, np.uint16), "instance_slots": (10, np.uint32)}
 
     def set_transforms(self, first: int, object_to_world, scales=None) -> None:
         """Replaces transforms first.. (object-to-world 4x4 matrices, as

@@ -1652,6 +1652,8 @@ long long ymrt_scene_download(const ymrt_scene* sc, int what, void* out, size_t 
     case YMRT_SCENE_LIGHT_TABLE: src = D.shape_light_table; bytes = sizeof(float) * D.shape_light_count; break;
     case YMRT_SCENE_INSTANCE_BUCKETS: src = D.inst_bucket; bytes = D.instance_count; break;
     case YMRT_SCENE_CAMERA_MEDIA: src = &D.camera.transfer; bytes = sizeof(RayTransfer); device = false; break;
+    case YMRT_SCENE_TLAS_KINDS: src = D.tlas_kinds; bytes = sizeof(uint16_t) * T.node_count; break;
+    case YMRT_SCENE_INSTANCE_SLOTS: src = D.inst_slots; bytes = sizeof(InstanceSlot) * D.instance_count; break;
     case YMRT_SCENE_FILE_INDEX:
       bytes = sizeof(uint32_t) * D.instance_count;
       if (T.prepared) src = T.file_idx[T.cur].ptr;

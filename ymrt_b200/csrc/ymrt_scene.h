@@ -272,25 +272,26 @@ YM_HD InstanceSlot make_instance_slot(uint32_t index, const Instance& inst, cons
 // 66 instances: backward 41.0 -> 36.3 ms, forward 25.5 -> 23.9; volumetric
 // 1280x720 16 spp, 10 instances, 232 -> 227). Children follow their parents in
 // the node order, so one pass from the last node up does it.
+//
+// One child's part: bit 0, it leads to a boundary instance; bit 8, to another.
+YM_HD uint32_t kinds_below(uint32_t node_kinds) {
+  return ((node_kinds & 0xFFu) ? 1u : 0u) | ((node_kinds >> 8) ? 1u << 8 : 0u);
+}
+YM_HD uint32_t leaf_kinds(const WideNode& w, int c, const uint32_t* prims, const Instance* instances) {
+  const uint32_t m = w.meta[c];
+  uint32_t kinds = 0;
+  for (uint32_t q = 0; q < (m >> 5); ++q)
+    kinds |= instances[prims[w.prim_base + (m & 31u) + q]].treat_as_boundary ? 1u : 1u << 8;
+  return kinds;
+}
 YM_HD void top_level_kinds(const WideNode* nodes, uint32_t n_nodes, const uint32_t* prims, const Instance* instances,
                            uint16_t* kinds) {
   for (uint32_t k = n_nodes; k-- > 0;) {
     const WideNode& w = nodes[k];
-    uint32_t boundary = 0, solid = 0;
-    for (int c = 0; c < 8; ++c) {
-      const uint32_t m = w.meta[c];
-      if ((w.imask >> c) & 1u) {
-        const uint32_t child = kinds[w.child_base + m];
-        if (child & 0xFFu) boundary |= 1u << c;
-        if (child >> 8) solid |= 1u << c;
-        continue;
-      }
-      for (uint32_t q = 0; q < (m >> 5); ++q) {
-        if (instances[prims[w.prim_base + (m & 31u) + q]].treat_as_boundary) boundary |= 1u << c;
-        else solid |= 1u << c;
-      }
-    }
-    kinds[k] = (uint16_t)(boundary | (solid << 8));
+    uint32_t v = 0;
+    for (int c = 0; c < 8; ++c)
+      v |= (((w.imask >> c) & 1u) ? kinds_below(kinds[w.child_base + w.meta[c]]) : leaf_kinds(w, c, prims, instances)) << c;
+    kinds[k] = (uint16_t)v;
   }
 }
 
