@@ -510,7 +510,8 @@ int ymrt_debug_bound_record(ymrt_context* ctx, uint32_t* words, size_t n_words, 
  * the context usable); 0 stops it. */
 void ymrt_debug_fail_allocations(int count);
 /* What a context has done, for tests of its bounds: out receives the first n
- * of: wave loops captured so far, captured loops kept. Returns how many there are. */
+ * of: wave loops captured so far, captured loops kept, waves of the last batch
+ * whose continuing rays were grouped. Returns how many there are. */
 int ymrt_debug_counters(const ymrt_context* ctx, uint64_t* out, size_t n);
 int ymrt_debug_occluded(ymrt_scene* scene, int n, const float* origin, const float* dir, const float* tmax,
                         int* occluded);

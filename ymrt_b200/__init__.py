@@ -207,7 +207,7 @@ class Context:
         _check(library().ymrt_get_option(self.h, OPTIONS[name], ctypes.byref(v)))
         return v.value
 
-    COUNTERS = ("loops_captured", "loops_kept")
+    COUNTERS = ("loops_captured", "loops_kept", "grouped_waves")
 
     def counters(self) -> dict:
         """What the context has done (ymrt_debug_counters)."""

@@ -531,6 +531,7 @@ int ymrt_create(int device_ordinal, ymrt_context** out) {
     return ctx->cuda_fail(e, "cudaMallocHost");
   if ((e = cudaMallocHost(&ctx->ctl_host, sizeof(WaveControl))) != cudaSuccess)
     return ctx->cuda_fail(e, "cudaMallocHost");
+  std::memset(ctx->ctl_host, 0, sizeof(WaveControl));
   if ((e = ctx->counters_buf.ensure(sizeof(WaveCounters))) != cudaSuccess) return ctx->cuda_fail(e, "cudaMalloc");
   *out = ctx.release();
   return YMRT_OK;
@@ -2420,7 +2421,7 @@ int ymrt_debug_occluded(ymrt_scene* sc, int n, const float* origin, const float*
 
 int ymrt_debug_counters(const ymrt_context* ctx, uint64_t* out, size_t n) {
   if (!ctx || (!out && n)) return YMRT_ERR_INVALID;
-  const uint64_t v[] = {ctx->loops_captured, ctx->graphs.size()};
+  const uint64_t v[] = {ctx->loops_captured, ctx->graphs.size(), ctx->ctl_host->grouped_waves};
   const size_t have = sizeof(v) / sizeof(v[0]);
   for (size_t k = 0; k < n; ++k) out[k] = k < have ? v[k] : 0u;
   return (int)have;

@@ -600,8 +600,9 @@ __global__ void __launch_bounds__(1024) k_ray_scan_blocks(const WaveControl* __r
   if (threadIdx.x == 0) H.ray_bins[2 * kRayBins + blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(1024) k_ray_scan_partials(const WaveControl* __restrict__ ctl, HitPool H) {
+__global__ void __launch_bounds__(1024) k_ray_scan_partials(WaveControl* ctl, HitPool H) {
   if (grouped_rays(ctl) == 0) return;
+  if (threadIdx.x == 0) ctl->grouped_waves += 1;
   const uint32_t k = threadIdx.x;
   const uint32_t v = k < kRayScanBlocks ? H.ray_bins[2 * kRayBins + k] : 0u;
   uint32_t total;

@@ -203,6 +203,7 @@ struct WaveControl {
   uint32_t max_waves;             // bound on waves (then YMRT_DEVERR_ITER)
   uint32_t more;                  // 1 while paths remain
   uint32_t scene_bits;            // bits of the scene's slot that lead the grouping's key
+  uint32_t grouped_waves;         // waves whose continuing rays were grouped
 };
 
 constexpr int kGradParams = 4;  // differentiated parameters per material: albedo r, g, b, roughness
