@@ -788,6 +788,8 @@ int ymrt_scene_upload(ymrt_context* ctx, const ymrt_host_scene* hs, const uint32
     return ctx->fail(YMRT_ERR_INVALID,
                      "halton permutation table must hold " + std::to_string(kHaltonTableSize) + " entries");
   const HostScene& s = hs->s;
+  if (s.tlas_prims.size() > kMaxInstanceSlots)
+    return ctx->fail(YMRT_ERR_UNSUPPORTED, "a scene of more than 2^28 instances");
   cudaSetDevice(ctx->device);
   std::unique_ptr<ymrt_scene> sc(new (std::nothrow) ymrt_scene());
   if (!sc) return YMRT_ERR_OOM;

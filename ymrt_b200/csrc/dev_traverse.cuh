@@ -40,6 +40,7 @@ constexpr int kMaxTraceBlock = 256;  // largest block k_extend and k_connect are
 // in bits 28-30 and the first one's leaf slot.
 constexpr uint32_t kInstanceEntry = 0x80000000u;
 constexpr uint32_t kEntryCountShift = 28, kEntrySlotMask = (1u << kEntryCountShift) - 1u;
+static_assert(kMaxInstanceSlots == kEntrySlotMask + 1u, "an entry holds any slot that a scene may have");
 
 struct TraversalStack {
   uint2* sh;  // shared-memory column of this thread: entry, entry distance (stride: the block's threads)

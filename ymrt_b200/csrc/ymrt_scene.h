@@ -254,6 +254,10 @@ struct alignas(16) InstanceSlot {
 };
 static_assert(sizeof(InstanceSlot) == 64, "InstanceSlot is four 16-byte words");
 constexpr uint32_t kSlotBoundary = 1, kSlotSphere = 2;
+// Leaf slots a top level may have: a traversal's stack entry holds a slot in 28
+// bits beside the count of its group (a scene of more is refused at upload:
+// its records alone would take 17 GB).
+constexpr uint32_t kMaxInstanceSlots = 1u << 28;
 YM_HD InstanceSlot make_instance_slot(uint32_t index, const Instance& inst, const mat4& world_to_object,
                                       const GeometryDesc& g) {
   InstanceSlot s;
