@@ -716,7 +716,10 @@ def cpu_baseline(path, perm, W, H, spp, depth, budget_s=10.0, threads=None, volu
     g++ -O3 -march, no query counters), on a bounded tile sample of the same
     frame, all host threads."""
     threads = threads or os.cpu_count() or 1
-    rs, (tb, te), rays, _ = _reference_sample(path, perm, W, H, spp, depth, budget_s, threads, volume)
+    try:
+        rs, (tb, te), rays, _ = _reference_sample(path, perm, W, H, spp, depth, budget_s, threads, volume)
+    except Exception as e:  # noqa: BLE001 - reported, not fatal for our own measurement
+        return {"unavailable": f"{type(e).__name__}: {e}"}
     rs.render_frame(1, tb, te, wave_capacity=256 * spp * min(te - tb, 64), threads=threads)
     secs = rs.last_render_seconds()
     isa = rs.isa
@@ -741,8 +744,11 @@ def run_reference(args):
     threads = os.cpu_count() or 1
     # each step a sample of about cpu_budget seconds, the whole run about two minutes at most
     budget = min(args.cpu_budget, 120.0 / (args.warmup + args.steps))
-    rs, (tb, te), rays_per_step, total_tiles = _reference_sample(path, perm, W, H, spp, wl["depth"], budget,
-                                                                 threads, wl.get("volume", False))
+    try:
+        rs, (tb, te), rays_per_step, total_tiles = _reference_sample(path, perm, W, H, spp, wl["depth"], budget,
+                                                                     threads, wl.get("volume", False))
+    except Exception as e:  # noqa: BLE001 - the reference's build is not here
+        return {"impl": "reference", "unavailable": f"{type(e).__name__}: {e}"}
     secs = 0.0
     for i in range(args.warmup + args.steps):
         # every step renders the same sample (frame 1 of those tiles), whose
