@@ -624,7 +624,7 @@ __device__ __forceinline__ void eval_chosen_light(const DeviceScene& S, const Ch
 // code, more than an SM's instruction caches hold, and warps left to run on
 // their own spread over all of it: they waited for instructions 21-32 of 28-40
 // cycles per issue. Behind barriers the warps of an SM run the same few KB at
-// a time, and the wait falls to 1-4 cycles. So the block is as wide as an SM
+// a time, and the wait falls to 1.3 (solid textures; surfaces 1.4). So the block is as wide as an SM
 // has registers for (512 threads of 128) where the code is widest: media and
 // textures (one B200, without barriers at 128 threads -> 512: volumetric
 // 1280x720 16 spp 528 -> 299 ms, solid textures 8 spp 197 -> 72 ms, image
